@@ -1,0 +1,64 @@
+"""Kernels and dispatch rules at the sizes where they can go wrong: edges of tiles, remainders,
+the smallest sizes, views that a cluster of blocks shares, against the FP64 oracle, the general
+path of the same library or an FP64 torch restatement.  Bar of the projectors and regularisers:
+1e-5 relative, as in the parity tests (32-bit sums)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tests import geometries as G
+from oracle import oracle as O
+from tigre_b200.utilities.geometry import cone_geometry
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def _geo(shape, det, pix, dso=1000.0, dsd=1536.0, offsets=False, mode="cone"):
+    g = cone_geometry(shape, [float(s) for s in shape], det, (pix, pix), DSO=dso, DSD=dsd)
+    g.mode = mode
+    if offsets:
+        g.offOrigin = np.array((1.5, -2.0, 3.25))
+        g.offDetector = np.array((2.4, -1.6))
+        g.COR = 0.7
+    return g
+
+
+def _plan(geo, ang):
+    from tigre_b200 import _native as N
+    return N.Plan(N.checked_geometry(geo, ang), 0)
+
+
+def _close(got, ref, tol=TOL):
+    mx, l2 = G.rel_err(got, ref)
+    assert mx <= tol and l2 <= tol, (mx, l2)
+
+
+# ------------------------------------------------------- backprojection: views over a cluster --
+@pytest.mark.parametrize("shape,views", [
+    ((64, 64, 64), 33),      # 16 tiles: 8 blocks share 33 views (4 or 5 each)
+    ((65, 17, 33), 16),      # ragged tiles in every axis, 4 blocks of 4 views
+    ((5, 3, 2), 9),          # one tile, odd views over 2 blocks
+    ((20, 40, 36), 7),       # too few views to share
+])
+@pytest.mark.parametrize("kind", ["FDK", "matched"])
+def test_backprojection_with_shared_views(shape, views, kind):
+    import torch
+    from tigre_b200 import _native as N, projectors as P
+    geo = _geo(shape, (40, 52), 2.0)
+    ang = G.angles(views)
+    proj = np.random.default_rng(views).random((views, 40, 52), dtype=np.float32)
+    plan = _plan(geo, ang)
+    d = torch.from_numpy(proj).cuda()
+    ref = O.atb(proj, geo, ang, kind)
+    got = P.atb(d, plan, kind)
+    _close(got.cpu().numpy(), ref)
+    assert torch.equal(got, P.atb(d, plan, kind))            # a fixed order of the sums
+    half = P.atb(d, plan, kind, out_dtype=torch.bfloat16).float().cpu().numpy()
+    _close(half, ref, 2.0 ** -8)                              # one rounding to BF16
+    N.check(N.lib().tigre_atb_ex(plan.handle, C.c_void_p(d.data_ptr()), N.F32, C.c_void_p(got.data_ptr()), N.F32,
+                                 P.BACKPROJECTORS[kind], 0, views, 1, None), "tigre_atb_ex")
+    _close(got.cpu().numpy(), 2.0 * ref)                      # accumulation
+    assert plan.status() == 0

@@ -28,8 +28,15 @@
 //    barrier or shared flag for this (measured: either costs 2-3 %).
 // A (block, view) whose footprint does not fit the box (possible for strongly
 // magnified geometries) falls back to bounds-checked global loads.
+//
+// Small volumes give few blocks (64^3: 16 for 148 SMs), each serially over all views, so the
+// views of a tile are then divided over a cluster of 2, 4 or 8 blocks (bp_splits): every block
+// sums its share of the views in registers as above, leaves the sums in shared memory, and each
+// adds up and writes its part of the tile's slices through distributed shared memory, in
+// a fixed order.  No workspace, no second launch, one rounding to the storage type.
 
 #include <type_traits>
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -43,6 +50,7 @@ namespace {
 
 constexpr int TXY = kBpTile;   // columns per block edge
 constexpr int VZ = kBpSlices;  // slices per thread
+constexpr int kMaxSplit = 8;   // blocks per tile at most: the portable cluster size
 constexpr unsigned kWaitLimit = 1u << 16;   // ~ a few ms with the back-off below
 
 struct BPKArgs {
@@ -58,6 +66,7 @@ struct BPKArgs {
     float scale;
     int accumulate;       // add into the existing volume instead of overwriting it
     int skip_view;        // failure-detection test: no copy is issued for this local view (-1: none)
+    int nsplit;           // blocks (one cluster) that share a tile's views
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -193,11 +202,16 @@ __device__ __forceinline__ float global_sample(const BPKArgs& p, const TP* P, fl
     return fmaf(av, a1 - a0, a0);
 }
 
-template <typename TP, typename TV, bool MATCHED, bool AXIAL>
+template <typename TP, typename TV, bool MATCHED, bool AXIAL, bool SPLIT>
 __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, BPKArgs p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ int info[2][4];
+    __shared__ int tile_failed;   // SPLIT: a wait of this block expired
+    // SPLIT: the blocks of a cluster (along z) own one tile and views [lb, lb + nviews) of it each
+    const int rank = SPLIT ? (int)(blockIdx.z % (unsigned)p.nsplit) : 0;
+    const int lb = SPLIT ? (int)((long)p.na * rank / p.nsplit) : 0;
+    const int nviews = (SPLIT ? (int)((long)p.na * (rank + 1) / p.nsplit) : p.na) - lb;
     // TMA destinations: 128-byte aligned, each buffer rounded up to 128 bytes
     const uint32_t base_off = (128u - (smem_u32(smem_raw) & 127u)) & 127u;
     const size_t buf_bytes = ((size_t)p.BU * p.BV * sizeof(TP) + 127) / 128 * 128;
@@ -210,7 +224,8 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
     // slice fall on a compact set of detector texels (few shared-memory wavefronts)
     const int wid = tid >> 5, ln = tid & 31;
     const int tx = (wid & 1) * 8 + (ln & 7), ty = (wid >> 1) * 4 + (ln >> 3);
-    const int x0 = blockIdx.x * TXY, y0 = blockIdx.y * TXY, z0 = blockIdx.z * VZ;
+    const int x0 = blockIdx.x * TXY, y0 = blockIdx.y * TXY;
+    const int z0 = (int)(SPLIT ? blockIdx.z / (unsigned)p.nsplit : blockIdx.z) * VZ;
     const int x = x0 + tx, y = y0 + ty;
     const bool active = x < p.nX && y < p.nY;
     const uint32_t bar0 = smem_u32(&bars[0]), bar1 = smem_u32(&bars[1]);
@@ -218,23 +233,25 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tile_failed = 0;
     }
     __syncthreads();
     if (tid < 32) {
-        plan_patch<TP>(p, &tmap, 0, x0, y0, z0, buf0, bar0, info[0], false);
-        if (p.na > 1) plan_patch<TP>(p, &tmap, 1, x0, y0, z0, buf1, bar1, info[1], false);
+        plan_patch<TP>(p, &tmap, lb, x0, y0, z0, buf0, bar0, info[0], false);
+        if (nviews > 1) plan_patch<TP>(p, &tmap, lb + 1, x0, y0, z0, buf1, bar1, info[1], false);
     }
     float acc[VZ];
 #pragma unroll
     for (int k = 0; k < VZ; ++k) acc[k] = 0.f;
     const TP* Pg = (const TP*)p.proj;
     const float pumax = (float)(p.BU - 2), pvmax = (float)(p.BV - 2);
-    int failed_at = -1;   // first view whose wait expired in this thread
-    for (int la = 0; la < p.na; ++la) {
-        const int s = la & 1;
+    int failed_at = -1;   // first view (of this block's) whose wait expired in this thread
+    for (int i = 0; i < nviews; ++i) {
+        const int la = lb + i;
+        const int s = i & 1;
         const uint32_t bar = s ? bar1 : bar0;
         // after one expired wait this thread waits no more (its sums are not written)
-        if (failed_at < 0 && !mbar_wait(bar, (uint32_t)((la >> 1) & 1))) failed_at = la;
+        if (failed_at < 0 && !mbar_wait(bar, (uint32_t)((i >> 1) & 1))) failed_at = i;
         const TP* patch = s ? buf1 : buf0;
         const uint32_t patch_u32 = s ? buf1_u32 : buf0_u32;
         const int u0 = info[s][0], v0 = info[s][1], fits = info[s][2];
@@ -390,14 +407,52 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
             }
         }
         __syncthreads();   // everyone is done with buffer s
-        if (tid < 32 && la + 2 < p.na) plan_patch<TP>(p, &tmap, la + 2, x0, y0, z0, s ? buf1 : buf0, bar, info[s], failed_at >= 0);
+        if (tid < 32 && i + 2 < nviews) plan_patch<TP>(p, &tmap, la + 2, x0, y0, z0, s ? buf1 : buf0, bar, info[s], failed_at >= 0);
     }
     if (tid == 0 && failed_at >= 0) {
         // thread 0 issued nothing after its failed view: the copies of that view and the next
         // may still be in flight, so wait for them (bounded) before the block's shared memory
         // is released
-        for (int v = failed_at; v < min(failed_at + 2, p.na); ++v)
-            if (v != p.skip_view) mbar_wait((v & 1) ? bar1 : bar0, (uint32_t)((v >> 1) & 1));
+        for (int v = failed_at; v < min(failed_at + 2, nviews); ++v)
+            if (lb + v != p.skip_view) mbar_wait((v & 1) ? bar1 : bar0, (uint32_t)((v >> 1) & 1));
+    }
+    if constexpr (SPLIT) {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        // this block's sums replace its patches (every warp is past the last view's barrier);
+        // a failed block still reaches both cluster barriers, and its tile is not written
+        float* sums = reinterpret_cast<float*>(smem_raw + base_off);   // [VZ][TXY * TXY]
+#pragma unroll
+        for (int k = 0; k < VZ; ++k) sums[k * TXY * TXY + tid] = acc[k];
+        if (failed_at >= 0) {
+            tile_failed = 1;
+            if (p.status) atomicOr(p.status, TIGRE_STATUS_WAIT_EXPIRED);
+        }
+        cluster.sync();
+        int bad = 0;
+#pragma unroll
+        for (int r = 0; r < kMaxSplit; ++r)
+            if (r < p.nsplit) bad |= *cluster.map_shared_rank(&tile_failed, r);
+        if (active && !bad) {
+            TV* V = (TV*)p.vol;
+            const int kend = min(VZ * (rank + 1) / p.nsplit, p.nZ - z0);
+#pragma unroll 2
+            for (int k = VZ * rank / p.nsplit; k < kend; ++k) {
+                // every block's value is requested before the first is used
+                float v[kMaxSplit];
+#pragma unroll
+                for (int r = 0; r < kMaxSplit; ++r)
+                    v[r] = r < p.nsplit ? cluster.map_shared_rank(sums, r)[k * TXY * TXY + tid] : 0.f;
+                float t = v[0];
+#pragma unroll
+                for (int r = 1; r < kMaxSplit; ++r) t += v[r];
+                const size_t i = ((size_t)(z0 + k) * p.nY + y) * p.nX + x;
+                const float o = p.accumulate ? to_f32<TV>(V[i]) : 0.f;
+                V[i] = from_f32<TV>(fmaf(t, p.scale, o));
+            }
+        }
+        cluster.sync();   // the sums stay until every block of the cluster has read them
+        return;
     }
     if (__any_sync(0xffffffffu, failed_at >= 0)) {
         if ((tid & 31) == 0 && p.status) atomicOr(p.status, TIGRE_STATUS_WAIT_EXPIRED);
@@ -429,18 +484,64 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
+// Blocks per tile, a power of two up to 8 (the portable cluster size), from the time that the
+// waves of resident blocks take: a view costs a block 3.8 us when two blocks share an SM and
+// 2.5 us alone (matched, 512^3 and 64^3), and a block 3 us to start and finish, about 8 us
+// with the exchange of the sums.  Sharing is taken where it saves 5 % in this account.  Matched,
+// one block per tile -> shared: 64^3 with 100 views 249 -> 62 us (8 blocks), 96^3 / 60 154 -> 106,
+// 128^3 / 180 445 -> 381, 160^3 / 90 547 -> 437; from 200^3 on the waves fill the chip by
+// themselves (200^3 / 90 measured 890 us alone and 904 us shared).
+int bp_splits(long blocks, int na) {
+    constexpr long kSms = 148, kSlots = 2 * kSms;
+    int best = 1;
+    double best_t = 0.0;
+    for (int s = 1; s <= kMaxSplit; s *= 2) {
+        if (s > 1 && na < 4 * s) break;
+        const int views = (na + s - 1) / s;
+        const long full = blocks * s / kSlots, rest = blocks * s % kSlots;
+        const double fixed = s == 1 ? 3.0 : 8.0;
+        double t = (double)full * (3.8 * views + fixed);
+        if (rest) t += (rest > kSms ? 3.8 : 2.5) * views + fixed;
+        if (s == 1 || t < 0.95 * best_t) { best = s; best_t = t; }
+    }
+    return best;
+}
+
 template <typename TP, typename TV>
-int launch_typed(const CUtensorMap& tm, const BPKArgs& a, bool matched, bool axial, cudaStream_t st) {
+int launch_typed(const CUtensorMap& tm, BPKArgs a, bool matched, bool axial, cudaStream_t st) {
     dim3 grid((a.nX + TXY - 1) / TXY, (a.nY + TXY - 1) / TXY, (a.nZ + VZ - 1) / VZ);
-    const size_t smem = 2 * (((size_t)a.BU * a.BV * sizeof(TP) + 127) / 128 * 128) + 128;
+    a.nsplit = bp_splits((long)grid.x * grid.y * grid.z, a.na);
+    size_t smem = 2 * (((size_t)a.BU * a.BV * sizeof(TP) + 127) / 128 * 128) + 128;
     auto go = [&](auto kern) -> int {
         TIGRE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kern<<<grid, TXY * TXY, smem, st>>>(tm, a);
         TIGRE_LAUNCHED();
         return TIGRE_SUCCESS;
     };
-    if (matched) return axial ? go(bp_tma_kernel<TP, TV, true, true>) : go(bp_tma_kernel<TP, TV, true, false>);
-    return axial ? go(bp_tma_kernel<TP, TV, false, true>) : go(bp_tma_kernel<TP, TV, false, false>);
+    auto go_split = [&](auto kern) -> int {
+        smem = std::max(smem, (size_t)VZ * TXY * TXY * sizeof(float) + 128);
+        TIGRE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = (unsigned)a.nsplit;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid.x, grid.y, grid.z * (unsigned)a.nsplit);
+        cfg.blockDim = dim3(TXY * TXY);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        TIGRE_CUDA(cudaLaunchKernelEx(&cfg, kern, tm, a));
+        TIGRE_LAUNCHED();
+        return TIGRE_SUCCESS;
+    };
+    if (a.nsplit > 1) {
+        if (matched) return axial ? go_split(bp_tma_kernel<TP, TV, true, true, true>) : go_split(bp_tma_kernel<TP, TV, true, false, true>);
+        return axial ? go_split(bp_tma_kernel<TP, TV, false, true, true>) : go_split(bp_tma_kernel<TP, TV, false, false, true>);
+    }
+    if (matched) return axial ? go(bp_tma_kernel<TP, TV, true, true, false>) : go(bp_tma_kernel<TP, TV, true, false, false>);
+    return axial ? go(bp_tma_kernel<TP, TV, false, true, false>) : go(bp_tma_kernel<TP, TV, false, false, false>);
 }
 
 }  // namespace
@@ -484,8 +585,6 @@ int launch_backproject_tma(TigrePlan* P, const void* proj, int pitch, int pdt, v
     a.skip_view = (skip >= 0 && skip < na) ? (int)skip : -1;
     const bool ax = P->axial;
     if (pdt == TIGRE_F32 && vdt == TIGRE_F32) return launch_typed<float, float>(tm, a, matched, ax, st);
-    if (pdt == TIGRE_BF16 && vdt == TIGRE_BF16) return launch_typed<__nv_bfloat16, __nv_bfloat16>(tm, a, matched, ax, st);
-    if (pdt == TIGRE_BF16 && vdt == TIGRE_F32) return launch_typed<__nv_bfloat16, float>(tm, a, matched, ax, st);
     if (pdt == TIGRE_F32 && vdt == TIGRE_BF16) return launch_typed<float, __nv_bfloat16>(tm, a, matched, ax, st);
     return fail(TIGRE_ERR_BAD_ASSERT, "unsupported dtype pair for the staged backprojector");
 }
