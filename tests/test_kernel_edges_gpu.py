@@ -62,3 +62,17 @@ def test_backprojection_with_shared_views(shape, views, kind):
                                  P.BACKPROJECTORS[kind], 0, views, 1, None), "tigre_atb_ex")
     _close(got.cpu().numpy(), 2.0 * ref)                      # accumulation
     assert plan.status() == 0
+
+
+# --------------------------------------------------------- backprojection: tilted frames --
+@pytest.mark.parametrize("shape", [(64, 16, 16), (65, 17, 18), (3, 30, 5), (130, 20, 33)])
+@pytest.mark.parametrize("kind", ["FDK", "matched"])
+def test_tilted_backprojection(shape, kind):
+    import torch
+    from tigre_b200 import projectors as P
+    geo = _geo(shape, (150, 60), 1.6)
+    geo.rotDetector = np.array((0.03, -0.02, 0.05))
+    ang = G.angles(11, tilt=True)
+    proj = np.random.default_rng(1).random((11, 150, 60), dtype=np.float32)
+    got = P.atb(torch.from_numpy(proj).cuda(), _plan(geo, ang), kind).cpu().numpy()
+    _close(got, O.atb(proj, geo, ang, kind))

@@ -109,6 +109,13 @@ __device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 t) {
     return __ffma2_rn(t, __ffma2_rn(a, f2(-1.f), b), a);
 }
 
+// 1 / a by the hardware's approximation (relative error below 2^-22)
+__device__ __forceinline__ float rcp_approx(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
 // texel-space (u - 0.5, v - 0.5) projection of voxel (x, y, z) for view frame F
 __device__ __forceinline__ void project_texel(const FrameBPK& F, float x, float y, float z, float& ub, float& vb) {
     const double vx = fma((double)z, F.dz[0], fma((double)y, F.dy[0], fma((double)x, F.dx[0], F.b[0])));
@@ -175,18 +182,6 @@ __device__ __forceinline__ void plan_patch(const BPKArgs& p, const CUtensorMap* 
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
         }
     }
-}
-
-template <typename TP>
-__device__ __forceinline__ float patch_sample(const TP* patch, int BU, int iu, float fu, float pv, float pvmax) {
-    pv = fminf(fmaxf(pv, 0.f), pvmax);
-    const int iv = (int)pv;
-    const float fv = pv - (float)iv;
-    const TP* r0 = patch + iv * BU + iu;
-    const float p00 = to_f32<TP>(r0[0]), p01 = to_f32<TP>(r0[1]);
-    const float p10 = to_f32<TP>(r0[BU]), p11 = to_f32<TP>(r0[BU + 1]);
-    const float a0 = fmaf(fu, p01 - p00, p00), a1 = fmaf(fu, p11 - p10, p10);
-    return fmaf(fv, a1 - a0, a0);
 }
 
 template <typename TP>
@@ -377,32 +372,94 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
                     }
                 }
             } else {
+                // Tilted frames: u, v and the depth all change along a column, so each voxel has
+                // its own reciprocal (hardware approximation and one Newton step) and horizontal
+                // fraction; otherwise the packed arithmetic of the axial path, two slices at
+                // a time.  The projective map keeps the order along a column, so when both of its
+                // ends fall inside the patch all of it does and no coordinate is clamped.
+                // 181 x 203 x 190 voxels, 77 views of 233 x 251, matched: 4218 -> 1170 us (an IEEE division,
+                // clamps, an unpacked sample and 90 instructions per voxel before); bound by issue.
                 const float dzx = (float)F.dz[0], dzy = (float)F.dz[1], dzz = (float)F.dz[2];
+                if (fits) {
+                    const float cup = F.cu - 0.5f - (float)u0, cvp = F.cv - 0.5f - (float)v0;   // patch coordinates
+                    constexpr uint32_t ES = (uint32_t)sizeof(TP);
+                    const uint32_t base = patch_u32 - 0x4B400000u * rowb - 0x4B400000u * ES;
+                    const float cw = 0.5f + (float)u0, cz = 0.5f + (float)v0;
+                    const float day0 = fmaf(cw, F.ddu, F.du0), dz0 = fmaf(cz, F.ddv, F.dzc);
+                    const float dx0 = F.daxc - F.rsx, dy0 = -F.daxs - F.rsy;
+                    const float rz0 = fmaf((float)z0, p.dVZ, F.rv0z);
+                    bool inside = true;
 #pragma unroll
-                for (int k = 0; k < VZ; ++k) {
-                    const float kf = (float)k;
-                    const float ex = fmaf(kf, dzx, vx), ey = fmaf(kf, dzy, vy), ez = fmaf(kf, dzz, vz);
-                    const float t = F.tnum / ex;
-                    const float u = fmaf(ey, t, F.cu), vtex = fmaf(ez, t, F.cv);
-                    float smp;
-                    if (fits) {
-                        const float pu = fminf(fmaxf(u - 0.5f - (float)u0, 0.f), pumax);
-                        const int iu = (int)pu;
-                        smp = patch_sample<TP>(patch, p.BU, iu, pu - (float)iu, vtex - 0.5f - (float)v0, pvmax);
-                    } else {
-                        smp = global_sample<TP>(p, Pg + (long)la * p.pitch * p.nV, u - 0.5f, vtex - 0.5f);
+                    for (int e = 0; e < 2; ++e) {
+                        const float kf = e ? (float)(VZ - 1) : 0.f;
+                        const float ex = fmaf(kf, dzx, vx), t = __fdividef(F.tnum, ex);
+                        const float ue = fmaf(fmaf(kf, dzy, vy), t, cup), ve = fmaf(fmaf(kf, dzz, vz), t, cvp);
+                        inside = inside && t > 0.f && ue >= 0.25f && ue <= pumax - 0.25f && ve >= 0.25f && ve <= pvmax - 0.25f;
                     }
-                    float w = wcol;
-                    if (MATCHED) {
-                        const float day = fmaf(u, F.ddu, F.du0);
-                        const float dx = fmaf(day, F.sina, F.daxc), dy = fmaf(day, F.cosa, -F.daxs);
-                        const float dz = fmaf(vtex, F.ddv, F.dzc);
-                        const float L2 = (F.rsx - dx) * (F.rsx - dx) + (F.rsy - dy) * (F.rsy - dy) + dz * dz;
-                        const float rvz = fmaf((float)(z0 + k), p.dVZ, F.rv0z);
-                        const float lsq = fmaf(rvz, rvz, cxy);
-                        w = L2 * (L2 * rsqrtf(L2)) * __frcp_rn(F.dsd * lsq);
+                    auto pairs = [&](auto clamp_tag) {
+                        constexpr bool CLAMP = decltype(clamp_tag)::value;
+#pragma unroll
+                        for (int k = 0; k < VZ; k += 2) {
+                            const float2 kk = f2((float)k, (float)(k + 1));
+                            const float2 ex = __ffma2_rn(kk, f2(dzx), f2(vx));
+                            float2 r = f2(rcp_approx(ex.x), rcp_approx(ex.y));
+                            r = __ffma2_rn(__ffma2_rn(neg2(ex), r, f2(1.f)), r, r);
+                            const float2 t = __fmul2_rn(f2(F.tnum), r);
+                            float2 pu = __ffma2_rn(__ffma2_rn(kk, f2(dzy), f2(vy)), t, f2(cup));
+                            float2 pv = __ffma2_rn(__ffma2_rn(kk, f2(dzz), f2(vz)), t, f2(cvp));
+                            if (CLAMP) {
+                                pu.x = fminf(fmaxf(pu.x, 0.f), pumax);
+                                pu.y = fminf(fmaxf(pu.y, 0.f), pumax);
+                                pv.x = fminf(fmaxf(pv.x, 0.f), pvmax);
+                                pv.y = fminf(fmaxf(pv.y, 0.f), pvmax);
+                            }
+                            // floors and fractions as on the axial path, for both coordinates
+                            const float2 tu = __fadd2_rz(pu, f2(12582912.0f)), tv = __fadd2_rz(pv, f2(12582912.0f));
+                            const float2 fu = __ffma2_rn(__fadd2_rn(tu, f2(-12582912.0f)), f2(-1.f), pu);
+                            const float2 fv = __ffma2_rn(__fadd2_rn(tv, f2(-12582912.0f)), f2(-1.f), pv);
+                            const uint32_t aa = (uint32_t)__float_as_int(tv.x) * rowb + ((uint32_t)__float_as_int(tu.x) * ES + base);
+                            const uint32_t ab = (uint32_t)__float_as_int(tv.y) * rowb + ((uint32_t)__float_as_int(tu.y) * ES + base);
+                            const float2 r0 = f2(lds<TP>(aa), lds<TP>(ab)), r0r = f2(lds<TP>(aa + ES), lds<TP>(ab + ES));
+                            const float2 r1 = f2(lds<TP>(aa + rowb), lds<TP>(ab + rowb));
+                            const float2 r1r = f2(lds<TP>(aa + rowb + ES), lds<TP>(ab + rowb + ES));
+                            const float2 smp = lerp2(lerp2(r0, r0r, fu), lerp2(r1, r1r, fu), fv);
+                            float2 w = f2(wcol);
+                            if (MATCHED) {
+                                const float2 day = __ffma2_rn(pu, f2(F.ddu), f2(day0)), dz = __ffma2_rn(pv, f2(F.ddv), f2(dz0));
+                                const float2 dx = __ffma2_rn(day, f2(F.sina), f2(dx0)), dy = __ffma2_rn(day, f2(F.cosa), f2(dy0));
+                                const float2 L2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                                const float2 rvz = __ffma2_rn(kk, f2(p.dVZ), f2(rz0));
+                                const float2 q = __fmul2_rn(f2(F.dsd), __ffma2_rn(rvz, rvz, f2(cxy)));
+                                const float2 L3 = __fmul2_rn(__fmul2_rn(L2, f2(rsqrtf(L2.x), rsqrtf(L2.y))), L2);
+                                w = __fmul2_rn(L3, f2(rcp_approx(q.x), rcp_approx(q.y)));
+                            }
+                            const float2 acc2 = __ffma2_rn(smp, w, f2(acc[k], acc[k + 1]));
+                            acc[k] = acc2.x;
+                            acc[k + 1] = acc2.y;
+                        }
+                    };
+                    if (inside) pairs(std::false_type{});
+                    else pairs(std::true_type{});
+                } else {
+#pragma unroll
+                    for (int k = 0; k < VZ; ++k) {
+                        const float kf = (float)k;
+                        const float ex = fmaf(kf, dzx, vx), ey = fmaf(kf, dzy, vy), ez = fmaf(kf, dzz, vz);
+                        const float t = F.tnum / ex;
+                        const float u = fmaf(ey, t, F.cu), vtex = fmaf(ez, t, F.cv);
+                        const float smp = global_sample<TP>(p, Pg + (long)la * p.pitch * p.nV, u - 0.5f, vtex - 0.5f);
+                        float w = wcol;
+                        if (MATCHED) {
+                            const float day = fmaf(u, F.ddu, F.du0);
+                            const float dx = fmaf(day, F.sina, F.daxc), dy = fmaf(day, F.cosa, -F.daxs);
+                            const float dz = fmaf(vtex, F.ddv, F.dzc);
+                            const float L2 = (F.rsx - dx) * (F.rsx - dx) + (F.rsy - dy) * (F.rsy - dy) + dz * dz;
+                            const float rvz = fmaf((float)(z0 + k), p.dVZ, F.rv0z);
+                            const float lsq = fmaf(rvz, rvz, cxy);
+                            w = L2 * (L2 * rsqrtf(L2)) * __frcp_rn(F.dsd * lsq);
+                        }
+                        acc[k] = fmaf(smp, w, acc[k]);
                     }
-                    acc[k] = fmaf(smp, w, acc[k]);
                 }
             }
         }
