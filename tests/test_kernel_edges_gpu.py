@@ -76,3 +76,23 @@ def test_tilted_backprojection(shape, kind):
     proj = np.random.default_rng(1).random((11, 150, 60), dtype=np.float32)
     got = P.atb(torch.from_numpy(proj).cuda(), _plan(geo, ang), kind).cpu().numpy()
     _close(got, O.atb(proj, geo, ang, kind))
+
+
+# ---------------------------------------------------------------------------- regularisers --
+TV_SHAPES = [(1, 1, 1), (1, 24, 30), (2, 25, 31), (5, 23, 61), (40, 49, 29), (3, 1, 95), (67, 7, 2)]
+
+
+@pytest.mark.parametrize("shape", TV_SHAPES)
+def test_tv_descents(shape):
+    import torch
+    from tigre_b200 import projectors as P
+    rng = np.random.default_rng(5)
+    img = rng.random(shape, dtype=np.float32)
+    prior = rng.random(shape, dtype=np.float32)
+
+    def dev(a):
+        return torch.from_numpy(a.copy()).cuda()
+    _close(P.tv_pocs_(dev(img), 0.01, 3).cpu().numpy(), O.pocs_tv(img, 0.01, 3))
+    _close(P.tv_aw_pocs_(dev(img), 0.01, 3, 0.3).cpu().numpy(), O.aw_pocs_tv(img, 0.01, 3, 0.3))
+    if int(np.prod(shape)) > 1:      # PICCS divides by |g|, which is 0 for a single voxel
+        _close(P.tv_piccs_(dev(img), dev(prior), 0.01, 0.4, 3).cpu().numpy(), O.piccs_tv(img, prior, 0.01, 0.4, 3))

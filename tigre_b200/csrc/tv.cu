@@ -6,8 +6,8 @@
 // The reference runs gradientTV, a device copy, two reduction kernels, a host
 // synchronisation and three element-wise kernels per step (~48 B/voxel).
 // Here a step is two passes and no host round trip (~12 B/voxel):
-//   pass 1  tv_tiled_kernel<kTvOutNorm>    stencil -> g, sum g^2 (FP64, one atomic per block)
-//   pass 2  tv_tiled_kernel<kTvOutUpdate>  stencil again -> g, writes f - alpha g / |g|,
+//   pass 1  tv_march_kernel<kTvOutNorm>    stencil -> g, sum g^2 (FP64, one atomic per block)
+//   pass 2  tv_march_kernel<kTvOutUpdate>  stencil again -> g, writes f - alpha g / |g|,
 //                             reading |g|^2 from device memory (ping-pong buffers)
 // g is recomputed rather than stored: the stencil is cheap, the bytes are not.
 //
@@ -20,7 +20,6 @@
 #include <cstdlib>
 #include <mutex>
 #include <string>
-#include <type_traits>
 
 #include "tigre_internal.h"
 
@@ -75,229 +74,183 @@ struct TVStep {
 
 constexpr int kTvPocs = 0, kTvAw = 1, kTvPiccs = 2;
 
-// ---- tiled gradientTV: POCS-TV, AwTV and PICCS passes and the autograd gradient ----
+// ---- gradientTV in registers: POCS-TV, AwTV and PICCS passes and the autograd gradient ----
 //
-// A block owns a 32 x (8 ROWS) tile of (x, y) columns and marches down a chunk of kTvZC
-// slices.  Per slice it stages f with a one-voxel x/y halo in shared memory and computes, at
-// every tile point and at the tile's +x column and +y row, the backward differences
-// (dz, dy, dx), their weighted forms (nz, ny, nx) and r = 1 / (sqrt(nz dz + ny dy + nx dx) + eps)
-// -- unweighted for POCS-TV (gradientTV, GD_TV.cu:117-143), with w = exp(-(d / delta)^2) per
-// component for AwTV (GD_AwTV.cu:117-158).  The gradient at (x, y, z) (dftv, GD_TV.cu:135-140)
-// is then
+// At every point the backward differences (dz, dy, dx), their weighted forms (nz, ny, nx) and
+// r = 1 / (sqrt(nz dz + ny dy + nx dx) + eps) -- unweighted for POCS-TV (gradientTV,
+// GD_TV.cu:117-143), with w = exp(-(d / delta)^2) per component for AwTV (GD_AwTV.cu:117-158).
+// The gradient at (x, y, z) (dftv, GD_TV.cu:135-140) is then
 //     (nz + ny + nx) r  -  nx(x+1) r(x+1)  -  ny(y+1) r(y+1)  -  nz(z+1) r(z+1),
-// each norm and weight evaluated once per voxel instead of four times, each voxel read from
-// global memory once per slice (plus the halo), and no integer division per voxel.  The
-// differences are the reference's exactly; r uses the hardware reciprocal square root and
-// reciprocal, so each term carries a relative error of a few 1e-7 against the reference's
-// IEEE divisions.  Zero-filled staging reproduces the boundary rules: the zero slices below
-// z = 0 and above z = nz - 1 (POCS-TV, AwTV), zero differences across the -x / -y faces.
+// each norm and weight evaluated once per voxel.  The differences are the reference's exactly;
+// r uses the hardware reciprocal square root and reciprocal, so each term carries a relative
+// error of a few 1e-7 against the reference's IEEE divisions.
 // PICCS (PICCS.cu:117-154) runs on the bare image (no z difference at z = 0, no +z term at the
-// last slice, eps 1e-6) and stages two fields, f and f - prior, for
+// last slice, eps 1e-6) with two fields, f and f - prior, for
 // g = (1 - ratio) grad TV(f) + ratio grad TV(f - prior).
 //
-// Pipeline: staged slices live in a ring of three buffers and the (ny, nx, r) planes in two,
-// so one barrier per slice suffices; each thread fetches its staged elements three slices
-// ahead into registers, so global loads overlap the arithmetic of the slices before them.
-constexpr int kTvTX = 32, kTvZC = 32;   // tile width; slices per chunk (tile height: 8 rows per thread row)
-constexpr int kTvFX = kTvTX + 2;         // staged f: x0-1 .. x0+32 (and y0-1 .. y0+TY)
-constexpr int kTvQX = kTvTX + 1;         // difference points: x0 .. x0+32 (and y0 .. y0+TY)
+// A warp owns 30 x tv_rows(KIND) columns and marches down a chunk of slices with everything in
+// registers: each lane holds one x of rows y0-1 .. y0+R of the previous and the current slice
+// (the next one is being fetched), the x neighbours come by shuffle (lanes 0 and 31 only
+// supply them), the y ones are the lane's own rows, and the +z term completes a slice one
+// step later.  No shared memory and no barrier.  Coordinates outside the volume are clamped when
+// loading, which makes the differences across the -x / -y faces and the terms beyond the last
+// x / y index exactly 0; the zero slices below z = 0 and above z = nz - 1 (POCS-TV, AwTV) are
+// staged as zeros, and PICCS repeats its end slices there.
+//
+// Bound by instruction issue (256^3: 46 thread instructions per voxel at 66-69 % of the issue slots,
+// beyond the arithmetic the three shuffles, the addresses and the rows shared with the
+// neighbouring warp), on small volumes by the latency of the few steps.  Per step of two passes:
+// 512^3 473 us (shared-memory tiles with one barrier per slice: 1113), 301 x 333 x 317 123 us (272),
+// 64^3 14 us (58).  4, 6 or 8 rows per warp with 8, 6 or 5 blocks per SM: 481 / 484 / 497 us at 512^3.
+constexpr int kTvLanes = 30;   // output columns of a warp
+constexpr int kTvWarps = 4;    // warps of a block, neighbours in y (they share their edge rows in L1)
 constexpr int kTvOutNorm = 0, kTvOutUpdate = 1, kTvOutGrad = 2;
 
+// rows of a warp's tile.  PICCS, with two fields in registers, takes fewer.
+constexpr int tv_rows(int kind) { return kind == kTvPiccs ? 4 : 6; }
+constexpr int tv_blocks(int kind) { return kind == kTvPiccs ? 5 : 6; }   // resident blocks per SM that registers allow
+
 struct TvTiles {
-    int tx, ty, tz, ntiles;
+    int tx, ty, zc;   // tiles in x and (block) tiles in y, slices per chunk
+    unsigned blocks;
 };
 
-TvTiles tv_tiles(const TVDims& d, int rows) {
-    const int TY = 8 * rows;
-    TvTiles t{(d.nx + kTvTX - 1) / kTvTX, (d.ny + TY - 1) / TY, (d.nz + kTvZC - 1) / kTvZC, 0};
-    t.ntiles = t.tx * t.ty * t.tz;
+// Slices per chunk: the fewest steps over the rounds of resident blocks, a chunk of zc slices
+// taking zc + 1 steps and about half a step to start.
+TvTiles tv_tiles(const TVDims& d, int kind) {
+    const int span = tv_rows(kind) * kTvWarps;
+    const int tx = (d.nx + kTvLanes - 1) / kTvLanes, ty = (d.ny + span - 1) / span;
+    const long slots = 148L * tv_blocks(kind);
+    TvTiles t{tx, ty, 0, 0};
+    double best = 0.0;
+    for (int zc = 2; zc <= 128; zc += zc < 16 ? 1 : zc / 8) {
+        const long blocks = (long)tx * ty * ((d.nz + zc - 1) / zc);
+        const double cost = (double)((blocks + slots - 1) / slots) * (zc + 1.5);
+        if (t.zc == 0 || cost < best) { best = cost; t.zc = zc; t.blocks = (unsigned)blocks; }
+    }
     return t;
 }
 
-int tv_tiled_grid(const TvTiles& t) { return std::min(t.ntiles, 148 * 8); }
+__device__ __forceinline__ float tv_rsqrt(float a) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ float tv_rcp(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
 
-// rows of the tile each thread owns (1: 32 x 8 tiles, 2: 32 x 16).  PICCS, with two staged
-// fields, uses one row.
-int tv_rows(int kind) { return kind == kTvPiccs ? 1 : 2; }
-
-// 1 / (sqrt(s) + eps) for s >= 0
-__device__ __forceinline__ float tv_rnorm(float s, float eps) {
-    const float q = s > 0.f ? s * rsqrtf(s) : 0.f;
-    return __fdividef(1.f, q + eps);
+// 1 / (sqrt(s) + eps) for the squared norm s = wz dz + wy dy + wx dx >= 0.  The smallest normal
+// number in the sum keeps the reciprocal square root finite at s = 0; it changes no value of
+// r, since a root below 1e-15 vanishes beside eps.
+__device__ __forceinline__ float tv_rnorm(float wz, float wy, float wx, float dz, float dy, float dx, float eps) {
+    const float s = fmaf(wx, dx, fmaf(wz, dz, fmaf(wy, dy, 1.1754944e-38f)));
+    return tv_rcp(__fadd_rn(__fmul_rn(s, tv_rsqrt(s)), eps));
 }
 
 // OUT: kTvOutNorm adds sum g^2 (FP64, one atomic per block) into *sums; kTvOutUpdate writes
 // o = f - alpha g / sqrt(*sums + st.norm_eps) (GD_TV.cu:556-597); kTvOutGrad writes o = g.
-// ROWS: tile rows per thread.  KIND: kTvPocs, kTvAw or kTvPiccs.
-template <int OUT, int ROWS, int KIND>
-__global__ void __launch_bounds__(256, ROWS == 1 ? 4 : 3) tv_tiled_kernel(const float* __restrict__ f,
+// KIND: kTvPocs, kTvAw or kTvPiccs.  Off: type of the byte offsets within a slice (32 bits wherever a
+// slice is below 4 GB, so that a load is one instruction on the slice's uniform base).
+template <int OUT, int KIND, typename Off>
+__global__ void __launch_bounds__(32 * kTvWarps, tv_blocks(KIND)) tv_march_kernel(const float* __restrict__ f,
                                                                            float* __restrict__ o, TVDims d, TvTiles T,
                                                                            TVStep st, double* __restrict__ sums,
                                                                            float alpha) {
     constexpr bool HALO = KIND != kTvPiccs;
-    constexpr int NF = KIND == kTvPiccs ? 2 : 1;   // staged fields: f (and f - prior)
-    constexpr int TY = 8 * ROWS, FY = TY + 2, QY = TY + 1;
-    constexpr int FS = FY * kTvFX;            // one staged slice of one field
-    constexpr int NS = (FS + 255) / 256;      // staged elements per thread, slice and field
-    __shared__ float F[NF * 3 * FS];
-    // ny, nx and r of a staged slice (nz is needed only at a thread's own columns: registers)
-    __shared__ float Qy[NF][2][QY][kTvQX], Qx[NF][2][QY][kTvQX], Qr[NF][2][QY][kTvQX];
-    const int tid = threadIdx.x, lx = tid & 31, ly = tid >> 5;
+    constexpr int NF = KIND == kTvPiccs ? 2 : 1;   // fields: f (and f - prior)
+    constexpr int R = tv_rows(KIND);
+    const int lane = threadIdx.x & 31, wid = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const int bx = (int)(blockIdx.x % (unsigned)T.tx), bt = (int)(blockIdx.x / (unsigned)T.tx);
+    const int x = bx * kTvLanes + lane - 1, y0 = (bt % T.ty * kTvWarps + wid) * R;
+    const int z0 = bt / T.ty * T.zc, zend = min(z0 + T.zc, d.nz);   // slice zend supplies the +z term
+    const size_t plane = (size_t)d.nx * d.ny;
     const float eps = st.grad_eps, idl = st.inv_delta;
     float scale = 0.f;
     if (OUT == kTvOutUpdate) scale = (float)((double)alpha / sqrt(*sums + st.norm_eps));
-    const int plane = d.nx * d.ny;   // the host keeps nx * ny * nz below 2^31
-    // the +x column (qx = 32, qy = 0..TY) and the +y row (qy = TY) of difference points
-    const bool extra = tid < QY + kTvTX;
-    const int eqx = tid < QY ? kTvTX : tid - QY, eqy = tid < QY ? tid : TY;
     double acc = 0.0;
-    for (int t = blockIdx.x; t < T.ntiles; t += gridDim.x) {
-        const int bx = t % T.tx, rt = t / T.tx;
-        const int by = rt % T.ty, bz = rt / T.ty;
-        const int x0 = bx * kTvTX, y0 = by * TY, z0 = bz * kTvZC;
-        const int zend = min(z0 + kTvZC, d.nz);   // output slices z0 .. zend-1; slice zend supplies the +z term
-        // thread tid stages elements k = tid + 256 j (k < FS) of every slice; their in-slice
-        // offsets are fixed per tile (-1 outside the volume: zero)
-        int off[NS];
+    const int nrow = lane >= 1 && lane <= kTvLanes && x < d.nx ? min(R, d.ny - y0) : 0;   // rows this lane writes
+    // byte offsets in a slice of the rows y0-1 .. y0+R, clamped to the volume
+    const Off xc = (Off)min(max(x, 0), d.nx - 1);
+    Off off[R + 2];
 #pragma unroll
-        for (int j = 0; j < NS; ++j) {
-            const int k = tid + 256 * j;
-            const int fy = k / kTvFX, fx = k - fy * kTvFX;
-            const int xx = x0 - 1 + fx, yy = y0 - 1 + fy;
-            off[j] = (k < FS && xx >= 0 && xx < d.nx && yy >= 0 && yy < d.ny) ? yy * d.nx + xx : -1;
-        }
-        auto fetch = [&](int zz, float (&v)[NF][NS]) {
-            const bool zin = zz >= 0 && zz < d.nz;
+    for (int j = 0; j < R + 2; ++j) off[j] = ((Off)min(max(y0 + j - 1, 0), d.ny - 1) * (Off)d.nx + xc) * 4;
+    auto at = [](const float* p, Off b) { return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + b)); };
+    auto fetch = [&](int z, float (&v)[NF][R + 2]) {
+        if (HALO) {
+            if (z >= 0 && z < d.nz) {
+                const float* p = f + (size_t)z * plane;
 #pragma unroll
-            for (int j = 0; j < NS; ++j) {
-                const bool ok = zin && off[j] >= 0;
-                const int i = zz * plane + off[j];
-                v[0][j] = ok ? __ldg(f + i) : 0.f;
-                if (NF == 2) v[NF - 1][j] = ok ? __ldg(f + i) - __ldg(st.prior + i) : 0.f;
-            }
-        };
-        auto put = [&](int slot, const float (&v)[NF][NS]) {
-#pragma unroll
-            for (int c = 0; c < NF; ++c)
-#pragma unroll
-                for (int j = 0; j < NS; ++j)
-                    if (j + 1 < NS || tid + 256 * j < FS) F[(c * 3 + slot) * FS + tid + 256 * j] = v[c][j];
-        };
-        // weighted differences and reciprocal norm at point (qx, qy) of field c, slice slot sc
-        // over slot sp; zlow: the slice has a z difference (always with the zero halo slices)
-        auto qpoint = [&](int c, int qx, int qy, int sc, int sp, bool zlow, float& wz, float& wy, float& wx) {
-            const int k = (qy + 1) * kTvFX + qx + 1;
-            const float* Fc = F + (c * 3 + sc) * FS;
-            const float v = Fc[k];
-            const float dz = zlow ? v - F[(c * 3 + sp) * FS + k] : 0.f;
-            const float dy = y0 + qy > 0 ? v - Fc[k - kTvFX] : 0.f;
-            const float dx = x0 + qx > 0 ? v - Fc[k - 1] : 0.f;
-            if (KIND == kTvAw) {
-                const float tz = dz * idl, ty = dy * idl, tx = dx * idl;
-                wz = expf(-(tz * tz)) * dz;
-                wy = expf(-(ty * ty)) * dy;
-                wx = expf(-(tx * tx)) * dx;
+                for (int j = 0; j < R + 2; ++j) v[0][j] = at(p, off[j]);
             } else {
-                wz = dz; wy = dy; wx = dx;
+#pragma unroll
+                for (int j = 0; j < R + 2; ++j) v[0][j] = 0.f;
             }
-            return tv_rnorm(wz * dz + wy * dy + wx * dx, eps);
-        };
-        const int x = x0 + lx;
-        bool inside[ROWS];
-        int own[ROWS];
+        } else {
+            const size_t zl = (size_t)min(max(z, 0), d.nz - 1) * plane;
+            const float *p = f + zl, *q = st.prior + zl;
 #pragma unroll
-        for (int q = 0; q < ROWS; ++q) {
-            const int y = y0 + ly + 8 * q;
-            inside[q] = x < d.nx && y < d.ny;
-            own[q] = y * d.nx + x;
+            for (int j = 0; j < R + 2; ++j) {
+                v[0][j] = at(p, off[j]);
+                v[NF - 1][j] = v[0][j] - at(q, off[j]);
+            }
         }
-        // R[j]: registers holding a fetched slice; at relative step j the slice zz + 1 is in
-        // R[(j + 1) % 3] and slice zz + 3 is fetched into R[j % 3]
-        float R[3][NF][NS];
-        fetch(z0 - 1, R[0]);
-        put(0, R[0]);
-        fetch(z0, R[0]);
-        put(1, R[0]);
-        fetch(z0 + 1, R[1]);
-        fetch(z0 + 2, R[2]);
-        __syncthreads();
-        float part[NF][ROWS], fown[ROWS];
+    };
+    float part[NF][R];
+    // slice z: P, C and N hold slices z - 1, z and z + 1 (being fetched)
+    auto step = [&](int z, float (&P)[NF][R + 2], float (&C)[NF][R + 2], float (&N)[NF][R + 2]) {
+        if (z < zend) fetch(z + 1, N);
+        const int emit = z > z0 ? nrow : 0;   // rows of slice z - 1, complete with its +z neighbour's term
+        char* ob = OUT == kTvOutNorm ? nullptr : reinterpret_cast<char*>(o + ((size_t)z * plane - plane));
 #pragma unroll
-        for (int q = 0; q < ROWS; ++q) {
-            fown[q] = 0.f;
-#pragma unroll
-            for (int c = 0; c < NF; ++c) part[c][q] = 0.f;
-        }
-        // one slice: slots (SP, SC, SN) hold slices zz - 1, zz, zz + 1; QB is the difference buffer
-        auto step = [&](int zz, auto SPc, auto SCc, auto SNc, auto QBc, auto RPc) {
-            constexpr int SP = decltype(SPc)::value, SC = decltype(SCc)::value, SN = decltype(SNc)::value;
-            constexpr int QB = decltype(QBc)::value, RP = decltype(RPc)::value;
-            if (zz + 1 <= zend) put(SN, R[RP]);
-            if (zz + 3 <= zend) fetch(zz + 3, R[(RP + 2) % 3]);
-            const bool zlow = HALO || zz > 0;
-            float wz[NF][ROWS], r[NF][ROWS], wy[NF][ROWS], wx[NF][ROWS];
+        for (int j = 0; j <= R; ++j) {   // points of row y0 + j
+            float gc[NF];
 #pragma unroll
             for (int c = 0; c < NF; ++c) {
-#pragma unroll
-                for (int q = 0; q < ROWS; ++q) {
-                    const int qy = ly + 8 * q;
-                    r[c][q] = qpoint(c, lx, qy, SC, SP, zlow, wz[c][q], wy[c][q], wx[c][q]);
-                    Qy[c][QB][qy][lx] = wy[c][q]; Qx[c][QB][qy][lx] = wx[c][q]; Qr[c][QB][qy][lx] = r[c][q];
+                const float v = C[c][j + 1];
+                const float dz = v - P[c][j + 1], dy = v - C[c][j];
+                const float dx = v - __shfl_up_sync(0xffffffffu, v, 1);
+                float wz = dz, wy = dy, wx = dx;
+                if (KIND == kTvAw) {
+                    const float tz = dz * idl, ty = dy * idl, tx = dx * idl;
+                    wz = expf(-(tz * tz)) * dz;
+                    wy = expf(-(ty * ty)) * dy;
+                    wx = expf(-(tx * tx)) * dx;
                 }
-                if (extra) {
-                    float a, b, e;
-                    const float m = qpoint(c, eqx, eqy, SC, SP, zlow, a, b, e);
-                    Qy[c][QB][eqy][eqx] = b; Qx[c][QB][eqy][eqx] = e; Qr[c][QB][eqy][eqx] = m;
-                }
-            }
-            __syncthreads();
-            // without the halo there is no +z neighbour above the last slice
-            const bool zterm = HALO || zz < d.nz;
-#pragma unroll
-            for (int q = 0; q < ROWS; ++q) {
-                const int qy = ly + 8 * q;
-                if (zz > z0 && inside[q]) {   // slice zz-1 is complete with its +z neighbour's term
-                    float gc[NF];
-#pragma unroll
-                    for (int c = 0; c < NF; ++c) gc[c] = zterm ? part[c][q] - wz[c][q] * r[c][q] : part[c][q];
-                    const float g = NF == 2 ? fmaf(1.f - st.ratio, gc[0], st.ratio * gc[NF - 1]) : gc[0];
-                    if (OUT == kTvOutNorm) acc += (double)g * (double)g;
-                    else {
-                        const int i = (zz - 1) * plane + own[q];
-                        o[i] = OUT == kTvOutUpdate ? fmaf(-scale, g, fown[q]) : g;
-                    }
-                }
-                if (zz < zend && inside[q]) {
-#pragma unroll
-                    for (int c = 0; c < NF; ++c) {
-                        float g = (wz[c][q] + wy[c][q] + wx[c][q]) * r[c][q];
-                        if (x + 1 < d.nx) g -= Qx[c][QB][qy][lx + 1] * Qr[c][QB][qy][lx + 1];
-                        if (y0 + qy + 1 < d.ny) g -= Qy[c][QB][qy + 1][lx] * Qr[c][QB][qy + 1][lx];
-                        part[c][q] = g;
-                    }
-                    fown[q] = F[SC * FS + (qy + 1) * kTvFX + lx + 1];
+                const float r = tv_rnorm(wz, wy, wx, dz, dy, dx, eps);
+                if (j > 0) part[c][j - 1] = fmaf(-wy, r, part[c][j - 1]);   // the +y term of the row below
+                if (j < R) {
+                    const float rx = __shfl_down_sync(0xffffffffu, r, 1), wx1 = __shfl_down_sync(0xffffffffu, wx, 1);
+                    gc[c] = fmaf(-wz, r, part[c][j]);
+                    part[c][j] = fmaf(-wx1, rx, (wz + wy + wx) * r);
                 }
             }
-        };
-        using I0 = std::integral_constant<int, 0>;
-        using I1 = std::integral_constant<int, 1>;
-        using I2 = std::integral_constant<int, 2>;
-        // six relative steps bring the three slots, two buffers and three register sets back to
-        // their starting assignment
-        for (int zb = z0; zb <= zend; zb += 6) {
-            step(zb, I0{}, I1{}, I2{}, I0{}, I1{});
-            if (zb + 1 > zend) break;
-            step(zb + 1, I1{}, I2{}, I0{}, I1{}, I2{});
-            if (zb + 2 > zend) break;
-            step(zb + 2, I2{}, I0{}, I1{}, I0{}, I0{});
-            if (zb + 3 > zend) break;
-            step(zb + 3, I0{}, I1{}, I2{}, I1{}, I1{});
-            if (zb + 4 > zend) break;
-            step(zb + 4, I1{}, I2{}, I0{}, I0{}, I2{});
-            if (zb + 5 > zend) break;
-            step(zb + 5, I2{}, I0{}, I1{}, I1{}, I0{});
+            if (j == R) break;
+            if (j < emit) {
+                const float g = NF == 2 ? fmaf(1.f - st.ratio, gc[0], st.ratio * gc[NF - 1]) : gc[0];
+                if (OUT == kTvOutNorm) acc = fma((double)g, (double)g, acc);
+                else *reinterpret_cast<float*>(ob + off[j + 1]) = OUT == kTvOutUpdate ? fmaf(-scale, g, P[0][j + 1]) : g;
+            }
         }
-        __syncthreads();   // the next tile restages the ring
+    };
+    if (y0 < d.ny) {
+        float A[NF][R + 2], B[NF][R + 2], C[NF][R + 2];
+        fetch(z0 - 1, A);
+        fetch(z0, B);
+#pragma unroll
+        for (int c = 0; c < NF; ++c)
+#pragma unroll
+            for (int j = 0; j < R; ++j) part[c][j] = 0.f;
+        // three steps bring the register sets back to their starting roles
+        for (int z = z0; z <= zend; z += 3) {
+            step(z, A, B, C);
+            if (z + 1 > zend) break;
+            step(z + 1, B, C, A);
+            if (z + 2 > zend) break;
+            step(z + 2, C, A, B);
+        }
     }
     if (OUT == kTvOutNorm) {
         acc = block_sum(acc);
@@ -305,26 +258,20 @@ __global__ void __launch_bounds__(256, ROWS == 1 ? 4 : 3) tv_tiled_kernel(const 
     }
 }
 
-// launch one tiled pass with the tile shape of tv_rows(KIND)
 template <int OUT, int KIND>
-void launch_tv_tiled(const float* f, float* o, const TVDims& d, const TVStep& st, double* sums, float alpha,
-                     cudaStream_t s) {
-    const int rows = tv_rows(KIND);
-    const TvTiles T = tv_tiles(d, rows);
-    if constexpr (KIND != kTvPiccs) {
-        if (rows == 2) {
-            tv_tiled_kernel<OUT, 2, KIND><<<tv_tiled_grid(T), 256, 0, s>>>(f, o, d, T, st, sums, alpha);
-            return;
-        }
-    }
-    tv_tiled_kernel<OUT, 1, KIND><<<tv_tiled_grid(T), 256, 0, s>>>(f, o, d, T, st, sums, alpha);
+void launch_tv(const float* f, float* o, const TVDims& d, const TVStep& st, double* sums, float alpha, cudaStream_t s) {
+    const TvTiles T = tv_tiles(d, KIND);
+    if ((double)d.nx * d.ny < 1.0e9)
+        tv_march_kernel<OUT, KIND, unsigned><<<T.blocks, 32 * kTvWarps, 0, s>>>(f, o, d, T, st, sums, alpha);
+    else
+        tv_march_kernel<OUT, KIND, size_t><<<T.blocks, 32 * kTvWarps, 0, s>>>(f, o, d, T, st, sums, alpha);
 }
 
 // POCS-TV step parameters (GD_TV.cu): no prior, no weights, 1e-7 under the norm, 1e-8 per gradient
 constexpr TVStep kPocsStep{nullptr, 0.f, 0.f, 1e-7, 1e-8f};
 
 // sum_i |grad f_i| over the voxels and the zero halo slice above the last one
-// (whose gradient norm is |f(x,y,nz-1)|); its derivative is the gradient of tv_tiled_kernel.
+// (whose gradient norm is |f(x,y,nz-1)|); its derivative is the gradient of tv_march_kernel.
 __global__ void __launch_bounds__(256) tv_value_kernel(const float* __restrict__ f, TVDims d, double* __restrict__ out) {
     double s = 0.0;
     TV_FOR_EACH_VOXEL(d, d.nz + 1, x, y, z, i) {
@@ -355,7 +302,7 @@ int tigre_tv_gradient(const void* d_img, int dtype, float* d_grad, long nx, long
     if (dtype != TIGRE_F32) return fail(TIGRE_ERR_BAD_ASSERT, "TV kernels take float32 volumes");
     if (nx <= 0 || ny <= 0 || nz <= 0 || !d_img || !d_grad) return fail(TIGRE_ERR_BAD_ASSERT, "bad TV arguments");
     TVDims d{(int)nx, (int)ny, (int)nz};
-    launch_tv_tiled<kTvOutGrad, kTvPocs>((const float*)d_img, d_grad, d, kPocsStep, nullptr, 0.f, (cudaStream_t)stream);
+    launch_tv<kTvOutGrad, kTvPocs>((const float*)d_img, d_grad, d, kPocsStep, nullptr, 0.f, (cudaStream_t)stream);
     TIGRE_LAUNCHED();
     return TIGRE_SUCCESS;
 }
@@ -387,8 +334,8 @@ int tigre_tv_pocs(void* d_img, int dtype, long nx, long ny, long nz, float alpha
     float* cur = (float*)d_img;
     float* nxt = d_work;
     for (int it = 0; it < max_iter; ++it) {
-        launch_tv_tiled<kTvOutNorm, kTvPocs>(cur, nullptr, d, kPocsStep, sums + it, 0.f, st);
-        launch_tv_tiled<kTvOutUpdate, kTvPocs>(cur, nxt, d, kPocsStep, sums + it, alpha, st);
+        launch_tv<kTvOutNorm, kTvPocs>(cur, nullptr, d, kPocsStep, sums + it, 0.f, st);
+        launch_tv<kTvOutUpdate, kTvPocs>(cur, nxt, d, kPocsStep, sums + it, alpha, st);
         std::swap(cur, nxt);
     }
     if (cur != (float*)d_img) TIGRE_CUDA(cudaMemcpyAsync(d_img, cur, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
@@ -412,8 +359,8 @@ static int tv_descent(void* d_img, long nx, long ny, long nz, float alpha, int m
     float* cur = (float*)d_img;
     float* nxt = d_work;
     for (int it = 0; it < max_iter; ++it) {
-        launch_tv_tiled<kTvOutNorm, KIND>(cur, nullptr, d, stp, sums + it, 0.f, st);
-        launch_tv_tiled<kTvOutUpdate, KIND>(cur, nxt, d, stp, sums + it, alpha, st);
+        launch_tv<kTvOutNorm, KIND>(cur, nullptr, d, stp, sums + it, 0.f, st);
+        launch_tv<kTvOutUpdate, KIND>(cur, nxt, d, stp, sums + it, alpha, st);
         std::swap(cur, nxt);
     }
     if (cur != (float*)d_img) TIGRE_CUDA(cudaMemcpyAsync(d_img, cur, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
@@ -523,8 +470,8 @@ extern "C" int tigre_tv_pocs_noalloc(void* d_img, int dtype, long nx, long ny, l
     float* cur = (float*)d_img;
     float* nxt = d_work;
     for (int it = 0; it < max_iter; ++it) {
-        launch_tv_tiled<kTvOutNorm, kTvPocs>(cur, nullptr, d, kPocsStep, sums + it, 0.f, st);
-        launch_tv_tiled<kTvOutUpdate, kTvPocs>(cur, nxt, d, kPocsStep, sums + it, alpha, st);
+        launch_tv<kTvOutNorm, kTvPocs>(cur, nullptr, d, kPocsStep, sums + it, 0.f, st);
+        launch_tv<kTvOutUpdate, kTvPocs>(cur, nxt, d, kPocsStep, sums + it, alpha, st);
         std::swap(cur, nxt);
     }
     if (cur != (float*)d_img) TIGRE_CUDA(cudaMemcpyAsync(d_img, cur, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
