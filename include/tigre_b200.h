@@ -268,6 +268,11 @@ int tigre_tv_piccs(void* d_img, const void* d_prior, int dtype, long nx, long ny
 long long tigre_tv_denoise_work_floats(long nx, long ny, long nz);
 int tigre_tv_denoise(const float* d_src, float* d_dst, long nx, long ny, long nz, float lambda, const float* spacing,
                      int max_iter, float* d_work, void* stream);
+/* As tigre_tv_denoise with d_work of work_floats floats: from tigre_tv_denoise_fused_floats(nx, ny, nz)
+ * on each iteration is one pass over the volume instead of two (the same recurrences). */
+long long tigre_tv_denoise_fused_floats(long nx, long ny, long nz);
+int tigre_tv_denoise_ex(const float* d_src, float* d_dst, long nx, long ny, long nz, float lambda,
+                        const float* spacing, int max_iter, float* d_work, long long work_floats, void* stream);
 /* TV gradient (GD_TV.cu:117-143, single-device boundary rule) into d_grad (FP32). */
 int tigre_tv_gradient(const void* d_img, int dtype, float* d_grad, long nx, long ny, long nz, void* stream);
 /* TV value sum_i |grad f_i| consistent with tigre_tv_gradient; added into *d_out (FP64). */

@@ -96,3 +96,31 @@ def test_tv_descents(shape):
     _close(P.tv_aw_pocs_(dev(img), 0.01, 3, 0.3).cpu().numpy(), O.aw_pocs_tv(img, 0.01, 3, 0.3))
     if int(np.prod(shape)) > 1:      # PICCS divides by |g|, which is 0 for a single voxel
         _close(P.tv_piccs_(dev(img), dev(prior), 0.01, 0.4, 3).cpu().numpy(), O.piccs_tv(img, prior, 0.01, 0.4, 3))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 16, 30), (1, 17, 31), (9, 15, 62), (35, 33, 28)])
+@pytest.mark.parametrize("iters", [0, 1, 2, 7])
+def test_denoise_in_one_pass_per_iteration(shape, iters):
+    import torch
+    from tigre_b200 import _native as N
+    img = np.random.default_rng(6).random(shape, dtype=np.float32)
+    nz, ny, nx = shape
+    L = N.lib()
+    spacing = (C.c_float * 3)(1.0, 0.5, 2.0)
+    out = {}
+    for name, floats in (("two", L.tigre_tv_denoise_work_floats(nx, ny, nz)),
+                         ("one", L.tigre_tv_denoise_fused_floats(nx, ny, nz))):
+        src = torch.from_numpy(img).cuda()
+        work = torch.full((floats,), float("nan"), device="cuda")       # no state is read before it is written
+        for alias in (False, True):
+            dst = src if alias else torch.empty_like(src)
+            N.check(L.tigre_tv_denoise_ex(C.c_void_p(src.data_ptr()), C.c_void_p(dst.data_ptr()), nx, ny, nz, 5.0,
+                                          C.cast(spacing, C.c_void_p), iters, C.c_void_p(work.data_ptr()), floats,
+                                          None), "tigre_tv_denoise_ex")
+            torch.cuda.synchronize()
+            out[name, alias] = dst.cpu().numpy()
+    for key in out:
+        _close(out[key], out["two", False], 1e-6)                       # the same recurrences
+    rc = L.tigre_tv_denoise_ex(C.c_void_p(src.data_ptr()), C.c_void_p(src.data_ptr()), nx, ny, nz, 5.0, None, 1,
+                               C.c_void_p(work.data_ptr()), 1, None)
+    assert rc == 4 and "work space" in N.last_error()
