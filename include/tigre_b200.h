@@ -321,6 +321,14 @@ int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D
 int tigre_conv3d_bwd_weight(const void* d_x, const void* d_dy, float* d_dw, long D, long H, long W, long Cin,
                             long Cout, void* d_col, void* stream);
 
+/* The ReLU's and the bias's share of a convolution's backward pass: g = dy where y > 0 else 0
+ * (BF16, n voxels x C channels; not written when relu == 0), db[c] = sum of g (FP32).
+ * C % 8 == 0, C <= 2048; d_dy, d_y, d_g 16-byte aligned; d_work: tigre_conv3d_relu_grad_work(n, C)
+ * floats of scratch. */
+long long tigre_conv3d_relu_grad_work(long n, long C);
+int tigre_conv3d_relu_grad(const void* d_dy, const void* d_y, void* d_g, float* d_db, long n, long C, int relu,
+                           float* d_work, void* stream);
+
 /* Fused steps of the warm-start U-Net's inference pass (no reference counterpart), BF16
  * channels-last activations with FP32 arithmetic; buffers 16-byte aligned.
  * pool2: y (D/2, H/2, W/2, C) = 2x2x2 mean of x (D, H, W, C); even sizes, C % 8 == 0.

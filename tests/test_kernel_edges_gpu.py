@@ -124,3 +124,71 @@ def test_denoise_in_one_pass_per_iteration(shape, iters):
     rc = L.tigre_tv_denoise_ex(C.c_void_p(src.data_ptr()), C.c_void_p(src.data_ptr()), nx, ny, nz, 5.0, None, 1,
                                C.c_void_p(work.data_ptr()), 1, None)
     assert rc == 4 and "work space" in N.last_error()
+
+
+# ---------------------------------------------------------------------------- convolutions --
+def _conv64(x, w, cout):
+    import torch
+    k = w.double().view(cout, 3, 3, 3, -1).permute(0, 4, 1, 2, 3)
+    return torch.nn.functional.conv3d(x.double().permute(3, 0, 1, 2)[None], k, padding=1)
+
+
+@pytest.mark.parametrize("D,H,W,cin,cout", [
+    (1, 1, 1, 16, 16), (4, 4, 16, 16, 32), (5, 17, 9, 32, 16), (3, 15, 33, 48, 64), (9, 20, 8, 16, 48),
+])
+def test_convolution_and_its_gradients(D, H, W, cin, cout):
+    """Bars: BF16 rounding of the outputs (2^-9 each, 2.5e-3 in all), FP32 sums for the weight and
+    bias gradients (1e-5) given the kernel's own ReLU mask."""
+    import torch
+    from tigre_b200 import _native as N, warmstart
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    x = torch.randn((D, H, W, cin), device="cuda", generator=g).bfloat16().requires_grad_(True)
+    w = (0.1 * torch.randn((cout, 27 * cin), device="cuda", generator=g)).bfloat16().float().requires_grad_(True)
+    b = torch.randn(cout, device="cuda", generator=g).requires_grad_(True)
+    dy = torch.randn((D, H, W, cout), device="cuda", generator=g).bfloat16()
+    y = warmstart.conv3d(x, w, b, True)
+    y.backward(dy)
+    x5 = x.detach().double().requires_grad_(True)
+    w5 = w.detach().double().requires_grad_(True)
+    ref = _conv64(x5, w5, cout) + b.detach().double()[None, :, None, None, None]
+    masked = dy.double() * (y.detach() > 0)
+    ref.backward(masked.permute(3, 0, 1, 2)[None])
+
+    def rel(a, r):
+        return float((a.double() - r).norm() / r.norm().clamp_min(1e-30))
+    assert rel(y.detach(), ref.detach().relu()[0].permute(1, 2, 3, 0)) < 2.5e-3
+    assert rel(x.grad, x5.grad) < 2.5e-3
+    assert rel(w.grad, w5.grad) < 1e-5
+    assert rel(b.grad, masked.sum(dim=(0, 1, 2))) < 1e-5
+    assert N.lib().tigre_conv3d_status(1) == 0
+
+
+@pytest.mark.parametrize("relu", [0, 1])
+@pytest.mark.parametrize("n,c", [(1, 8), (1000, 24), (70, 2048), (4097, 16)])
+def test_relu_and_bias_gradient(n, c, relu):
+    """NaN, infinities and -0 go through as dy * (y > 0) gives them."""
+    import torch
+    from tigre_b200 import _native as N
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    dy = torch.randn((n, c), device="cuda", generator=g).bfloat16()
+    y = torch.randn((n, c), device="cuda", generator=g).bfloat16()
+    if n > 1:
+        dy[1, 0], dy[0, 1], y[0, 1] = float("nan"), float("inf"), -1.0
+    out, db = torch.empty_like(dy), torch.empty(c, device="cuda")
+    work = torch.empty(N.lib().tigre_conv3d_relu_grad_work(n, c), device="cuda")
+    N.check(N.lib().tigre_conv3d_relu_grad(C.c_void_p(dy.data_ptr()), C.c_void_p(y.data_ptr()),
+                                           C.c_void_p(out.data_ptr()), C.c_void_p(db.data_ptr()), n, c, relu,
+                                           C.c_void_p(work.data_ptr()), None),
+            "tigre_conv3d_relu_grad")
+    ref = dy.float() * (y > 0) if relu else dy.float()
+    if relu:
+        assert torch.equal(out.view(torch.int16)[~ref.isnan()], ref.bfloat16().view(torch.int16)[~ref.isnan()])
+        assert bool(out[ref.isnan()].isnan().all())
+    want = ref.double().sum(0)
+    fine = want.isfinite()
+    assert torch.equal(fine, db.isfinite())
+    # FP32 sums of n terms in a tree: relative to the sum of magnitudes
+    size = ref.abs().double().sum(0)
+    assert bool(((db.double() - want).abs() <= 1e-5 * size)[fine].all())

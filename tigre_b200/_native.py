@@ -127,6 +127,9 @@ _SIGS = {
                                       C.c_long, C.c_long, C.c_void_p]),
     "tigre_conv3d_fwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long,
                                    C.c_long, C.c_long, C.c_long, C.c_int, C.c_void_p, C.c_void_p]),
+    "tigre_conv3d_relu_grad_work": (C.c_longlong, [C.c_long, C.c_long]),
+    "tigre_conv3d_relu_grad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long, C.c_int,
+                                         C.c_void_p, C.c_void_p]),
     "tigre_conv3d_bwd_data": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long, C.c_long, C.c_long,
                                         C.c_long, C.c_void_p, C.c_void_p]),
     "tigre_conv3d_bwd_weight": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long, C.c_long, C.c_long,

@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cstdint>
 #include <mutex>
 
@@ -632,7 +633,8 @@ int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D
     return TIGRE_SUCCESS;
 }
 
-// dw (FP32, Cout x 27*Cin) += dy^T . col, with col = im2col(x) recomputed into d_col.
+// dw (FP32, Cout x 27*Cin) += dy^T . im2col(x): staged voxel tiles (conv3d_wgrad.cu) where both
+// channel counts are multiples of 16, else a GEMM over im2col(x) in d_col.
 int tigre_conv3d_bwd_weight(const void* d_x, const void* d_dy, float* d_dw, long D, long H, long W, long Cin,
                             long Cout, void* d_col, void* stream) {
     TIGRE_NVTX("tigre_conv3d_bwd_weight");
@@ -640,6 +642,10 @@ int tigre_conv3d_bwd_weight(const void* d_x, const void* d_dy, float* d_dw, long
         return fail(TIGRE_ERR_BAD_ASSERT, "bad conv3d arguments");
     const long M = D * H * W, K = 27 * Cin;
     cudaStream_t st = (cudaStream_t)stream;
+    if (conv_wgrad_supported(Cin, Cout) && (((uintptr_t)d_x | (uintptr_t)d_dy | (uintptr_t)d_col) & 15) == 0 &&
+        D < INT_MAX && H < INT_MAX && W < INT_MAX)
+        return launch_conv_wgrad((const __nv_bfloat16*)d_x, (const __nv_bfloat16*)d_dy, d_dw, D, H, W, Cin, Cout,
+                                 (float*)d_col, st);
     im2col_kernel<<<grid_for_conv(M * K), 256, 0, st>>>((const __nv_bfloat16*)d_x, (__nv_bfloat16*)d_col, (int)D,
                                                         (int)H, (int)W, (int)Cin);
     TIGRE_LAUNCHED();

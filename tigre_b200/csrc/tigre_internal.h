@@ -186,6 +186,9 @@ bool conv_tc_halo_supported(long D, long H, long W, long Cin, long Cout);
 int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias, __nv_bfloat16* yb,
                         float* yf, long D, long H, long W, long Cin, long Cout, int relu, int flip,
                         __nv_bfloat16* wk_scratch, int* status, cudaStream_t st);
+bool conv_wgrad_supported(long Cin, long Cout);
+int launch_conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw, long D, long H, long W, long Cin,
+                      long Cout, float* work, cudaStream_t st);
 int launch_backproject(TigrePlan* p, const void* proj_pad, int pdt, void* vol, int vdt, int matched, int a0, int a1,
                        int accumulate, cudaStream_t st);
 

@@ -100,22 +100,35 @@ def _conv_fn():
             x, wb, y = ctx.saved_tensors
             D, H, W, Cin = x.shape
             Cout = wb.shape[0]
-            g = dy.float()
-            if ctx.relu:
-                g = g * (y > 0)
-            db = g.sum(dim=(0, 1, 2))
-            gb = g.to(T.bfloat16).contiguous()
+            if dy.dtype == T.bfloat16 and Cout % 8 == 0 and Cout <= 2048 and dy.contiguous().data_ptr() % 16 == 0:
+                # ReLU mask and bias sums in one pass
+                dy = dy.contiguous()
+                gb = T.empty_like(dy) if ctx.relu else dy
+                db = T.empty(Cout, dtype=T.float32, device=x.device)
+                work = T.empty(int(N.lib().tigre_conv3d_relu_grad_work(D * H * W, Cout)), dtype=T.float32,
+                               device=x.device)
+                N.check(N.lib().tigre_conv3d_relu_grad(C.c_void_p(dy.data_ptr()), C.c_void_p(y.data_ptr()),
+                                                       C.c_void_p(gb.data_ptr()), C.c_void_p(db.data_ptr()), D * H * W,
+                                                       Cout, 1 if ctx.relu else 0, C.c_void_p(work.data_ptr()),
+                                                       _stream(x)), "tigre_conv3d_relu_grad")
+            else:
+                g = dy.float()
+                if ctx.relu:
+                    g = g * (y > 0)
+                db = g.sum(dim=(0, 1, 2))
+                gb = g.to(T.bfloat16).contiguous()
             L = N.lib()
-            dx = T.empty((D, H, W, Cin), dtype=T.float32, device=x.device)
             if Cout % 8 == 0:
+                dx = T.empty((D, H, W, Cin), dtype=T.bfloat16, device=x.device)
                 # the data gradient is the forward convolution of dy with the tap-flipped,
                 # channel-transposed weights: wt[c][t*Cout + co] = w[co][(26 - t)*Cin + c]
                 wt = wb.view(Cout, 27, Cin).flip(1).permute(2, 1, 0).reshape(Cin, 27 * Cout).contiguous()
                 col = _SCRATCH.get(int(L.tigre_conv3d_col_elems(D, H, W, Cout)), "col", x.device)
-                N.check(L.tigre_conv3d_fwd(C.c_void_p(gb.data_ptr()), C.c_void_p(wt.data_ptr()), None, None,
-                                           C.c_void_p(dx.data_ptr()), D, H, W, Cout, Cin, 0,
+                N.check(L.tigre_conv3d_fwd(C.c_void_p(gb.data_ptr()), C.c_void_p(wt.data_ptr()), None,
+                                           C.c_void_p(dx.data_ptr()), None, D, H, W, Cout, Cin, 0,
                                            C.c_void_p(col.data_ptr()), _stream(x)), "tigre_conv3d_fwd")
             else:
+                dx = T.empty((D, H, W, Cin), dtype=T.float32, device=x.device)
                 dcol = _SCRATCH.get(int(L.tigre_conv3d_col_elems(D, H, W, Cin)), "dcol", x.device)
                 N.check(L.tigre_conv3d_bwd_data(C.c_void_p(gb.data_ptr()), C.c_void_p(wb.data_ptr()),
                                                 C.c_void_p(dx.data_ptr()), D, H, W, Cin, Cout,
