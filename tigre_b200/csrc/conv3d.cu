@@ -505,7 +505,7 @@ int grid_for_conv(long n) { return (int)std::min<long>((n + 255) / 256, 148L * 3
 using namespace tigre;
 
 // Forward path selection: 3 (default) = the tcgen05 halo-tile kernel (conv3d_tc.cu) wherever its
-// shape rules hold (Cin % 16 == 0, Cout % 16 == 0, W % 8 == 0, H % 16 == 0), else mode 2;
+// shape rules hold (Cin % 16 == 0, Cout % 16 == 0), else mode 2;
 // 0 = warp-level implicit GEMM, 1 = tcgen05 implicit GEMM with per-step gathers, 2 = that
 // tcgen05 kernel for narrow layers (Cin <= 16 or Cout == 16) and the warp-level one for wider ones.
 static std::atomic<int> g_conv_tcgen05{3};
@@ -616,7 +616,7 @@ int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D
     const long M = D * H * W, K = 27 * Cin;
     cudaStream_t st = (cudaStream_t)stream;
     if (g_conv_tcgen05.load() == 3 && ((uintptr_t)d_dy & 15) == 0 && ((uintptr_t)d_dcol & 15) == 0 &&
-        conv_tc_halo_supported(D, H, W, Cout, Cin)) {
+        Cout <= 2 * M && conv_tc_halo_supported(D, H, W, Cout, Cin)) {   // d_dcol holds the arranged weights
         // the data gradient is the convolution of dy with the tap-flipped, channel-transposed
         // weights: the halo kernel, FP32 output, no im2col (d_dcol holds the arranged weights)
         return launch_conv_tc_halo((const __nv_bfloat16*)d_dy, (const __nv_bfloat16*)d_w, nullptr, nullptr, d_dx, D,

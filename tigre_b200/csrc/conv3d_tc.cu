@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_const
     __shared__ int abort_flag;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const uint32_t base = (su32(smem_raw) + 1023u) & ~1023u;
-    const int tiles_x = p.W / kTx, tiles_y = p.H / kTy;
+    const int tiles_x = (p.W + kTx - 1) / kTx, tiles_y = (p.H + kTy - 1) / kTy;
     const int bx = blockIdx.x % tiles_x, by = (blockIdx.x / tiles_x) % tiles_y, bz = blockIdx.x / (tiles_x * tiles_y);
     const int x0 = bx * kTx, y0 = by * kTy, z0 = bz * p.zt;
     const int N = p.Cout;
@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_const
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int r = 32 * wid + lane;          // accumulator row: 8 y + x
         const int x = x0 + (r & 7), y = y0 + (r >> 3);
-        for (int zl = 0; zl < p.zt; ++zl) {
+        const bool inside = x < p.W && y < p.H;   // a tile may reach past the volume's last x, y or z
+        for (int zl = 0; zl < p.zt && z0 + zl < p.D; ++zl) {
             const size_t vox = ((size_t)(z0 + zl) * p.H + y) * p.W + x;
             for (int c0 = 0; c0 < N; c0 += 16) {
                 uint32_t v[16];
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_const
                       "=r"(v[15])
                     : "r"(taddr));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (!inside) continue;
                 float f[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
@@ -296,7 +298,8 @@ static void conv_tc_shape(int N, int D, int nchunks, int* zt, int* stages, uint3
     for (int budget : {112 * 1024, 200 * 1024}) {
         for (int i = 0; i < 3; ++i) {
             const int z = cand[i];
-            if (D % z || (size_t)z * N > 512) continue;
+            // slices past the last one are computed for nothing: at most a quarter of them
+            if ((D + z - 1) / z * z * 4 > 5 * D || (size_t)z * N > 512) continue;
             const uint32_t tb = (uint32_t)(kHx * kHy * (z + 2) * kCC * 2), wb = (uint32_t)(27 * kCC * N * 2);
             const uint32_t stb = (tb + wb + 1023u) & ~1023u;
             for (int s = std::min(3, nchunks); s >= 1; --s) {
@@ -313,7 +316,7 @@ static void conv_tc_shape(int N, int D, int nchunks, int* zt, int* stages, uint3
 }
 
 bool conv_tc_halo_supported(long D, long H, long W, long Cin, long Cout) {
-    if (Cin % kCC || Cout % 16 || Cout < 16 || Cout > 256 || W % kTx || H % kTy) return false;
+    if (Cin % kCC || Cout % 16 || Cout < 16 || Cout > 256) return false;
     int zt, st;
     uint32_t tb, wb;
     conv_tc_shape((int)Cout, (int)D, (int)(Cin / kCC), &zt, &st, &tb, &wb);
@@ -371,7 +374,7 @@ int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* w, const fl
     const size_t floor_smem = max_ctas >= 8 ? 0 : (size_t)(233472 / (max_ctas + 1) - 1024 + 64);
     const size_t smem = std::max(need, floor_smem);
     TIGRE_CUDA(cudaFuncSetAttribute(conv_tc_halo_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const long ntiles = (W / kTx) * (H / kTy) * (D / zt);
+    const long ntiles = ((W + kTx - 1) / kTx) * ((H + kTy - 1) / kTy) * ((D + zt - 1) / zt);
     conv_tc_halo_kernel<3><<<(unsigned)ntiles, 128, smem, st>>>(tm, a);
     TIGRE_LAUNCHED();
     return TIGRE_SUCCESS;
