@@ -192,3 +192,27 @@ def test_relu_and_bias_gradient(n, c, relu):
     # FP32 sums of n terms in a tree: relative to the sum of magnitudes
     size = ref.abs().double().sum(0)
     assert bool(((db.double() - want).abs() <= 1e-5 * size)[fine].all())
+
+
+@pytest.mark.parametrize("c", [8, 16, 32])
+@pytest.mark.parametrize("D,H,W", [(1, 1, 1), (2, 8, 62), (17, 9, 65), (33, 7, 126)])
+def test_first_and_last_convolution(c, D, H, W):
+    """Bar: one BF16 rounding of the convolution's value (2^-8 of its size)."""
+    import torch
+    from tigre_b200 import _native as N
+    g = torch.Generator(device="cuda")
+    g.manual_seed(4)
+    L, p = N.lib(), lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    vol = torch.randn((D, H, W), device="cuda", generator=g)
+    w = torch.randn((c, 27), device="cuda", generator=g).bfloat16()
+    b = torch.randn(c, device="cuda", generator=g)
+    y = torch.empty((D, H, W, c), dtype=torch.bfloat16, device="cuda")
+    N.check(L.tigre_unet_conv_in(p(vol), p(w), p(b), p(y), D, H, W, c, 0, None), "conv_in")
+    ref = (_conv64(vol.bfloat16()[..., None], w, c) + b.double()[None, :, None, None, None])[0].permute(1, 2, 3, 0)
+    assert float((y.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max())
+    x = torch.randn((D, H, W, c), device="cuda", generator=g).bfloat16()
+    wo = torch.randn((1, 27 * c), device="cuda", generator=g).bfloat16()
+    out = torch.empty_like(vol)
+    N.check(L.tigre_unet_conv_out(p(x), c, p(wo), 0.25, p(vol), p(out), D, H, W, None), "conv_out")
+    ref = _conv64(x, wo, 1)[0, 0] + 0.25
+    assert float((out.double() - vol.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()) + 1e-6

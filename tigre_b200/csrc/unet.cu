@@ -12,6 +12,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "tigre_internal.h"
 
@@ -81,68 +82,238 @@ __global__ void up_concat_kernel(const uint4* __restrict__ low, int Ca8, const u
     }
 }
 
-// first convolution: one input channel (vol, FP32, rounded to BF16), Cout <= 32 outputs
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
+    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+}
+
+// First convolution: one input channel (vol, FP32, rounded to BF16), COUT outputs, as warp-level
+// m16n8k16 products of 16 voxels along x with the taps as K.  Per (dz, dy) row the three dx taps
+// take two K pairs, (x-1, x) and (x+1, -), so that an operand register is one 32-bit word of the
+// staged row; the row is kept twice, the second copy shifted by one voxel, which makes the pair of
+// any x an aligned word.  18 of 24 K pairs carry weights; the others and the unused halves are
+// zeroed on both sides.  A block marches a 64 x 8 tile of (x, y) down kInZ slices, three staged at a
+// time; output column c of tile t is channel 2 NT (c / 2) + 2 t + c % 2, so a thread stores
+// 4 NT contiguous bytes.
+// 256^3, 16 channels: 205 us, 604 MB written and read at 2.9 TB/s (scalar FMAs, 27 bounds-tested loads a
+// voxel: 806 us); bound by the shared-memory loads of the operands and the staging.
+constexpr int kInX = 64, kInY = 8, kInZ = 16;
+constexpr int kInWords = kInX / 2 + 2;                 // words of one staged row and copy
+constexpr int kInPitch = 2 * kInWords + 1;             // both copies (odd: rows fall in other banks)
+
 template <int COUT>
 __global__ void __launch_bounds__(256) conv_in_kernel(const float* __restrict__ vol, const __nv_bfloat16* __restrict__ w,
                                                       const float* __restrict__ b, __nv_bfloat16* __restrict__ y,
-                                                      int D, int H, int W, int relu) {
-    __shared__ float sw[27][COUT];
-    __shared__ float sb[COUT];
-    for (int i = threadIdx.x; i < 27 * COUT; i += blockDim.x) sw[i % 27][i / 27] = __bfloat162float(w[i]);
-    for (int i = threadIdx.x; i < COUT; i += blockDim.x) sb[i] = b ? b[i] : 0.f;
-    __syncthreads();
-    const long total = (long)D * H * W;
-    for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < total; v += (long)gridDim.x * blockDim.x) {
-        const int x = (int)(v % W), yy = (int)((v / W) % H), z = (int)(v / ((long)W * H));
-        float acc[COUT];
+                                                      int D, int H, int W, int tx, int ty, int relu) {
+    constexpr int NT = COUT / 8;
+    __shared__ uint32_t ring[3][kInY + 2][kInPitch];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q = lane & 3;
+    const int bx = (int)(blockIdx.x % (unsigned)tx), bt = (int)(blockIdx.x / (unsigned)tx);
+    const int x0 = bx * kInX, y0 = bt % ty * kInY, z0 = bt / ty * kInZ, zend = min(z0 + kInZ, D);
+    auto channel = [](int t, int c) { return 2 * NT * (c >> 1) + 2 * t + (c & 1); };
+    // weights: K pair slot s = 8 kstep + 4 half + q holds taps (2 (s % 2), 2 (s % 2) + 1) of row s / 2
+    uint32_t wb[3][2][NT];
+    float bias[NT][2];
 #pragma unroll
-        for (int c = 0; c < COUT; ++c) acc[c] = sb[c];
+    for (int t = 0; t < NT; ++t) {
 #pragma unroll
-        for (int t = 0; t < 27; ++t) {
-            const int sx = x + t % 3 - 1, sy = yy + (t / 3) % 3 - 1, sz = z + t / 9 - 1;
-            float in = 0.f;
-            if (sx >= 0 && sx < W && sy >= 0 && sy < H && sz >= 0 && sz < D)
-                in = __bfloat162float(__float2bfloat16(__ldg(vol + ((long)sz * H + sy) * W + sx)));
+        for (int k = 0; k < 3; ++k)
 #pragma unroll
-            for (int c = 0; c < COUT; ++c) acc[c] = fmaf(sw[t][c], in, acc[c]);
+            for (int h = 0; h < 2; ++h) {
+                const int s = 8 * k + 4 * h + q, row = s >> 1;
+                const __nv_bfloat16* src = w + channel(t, g) * 27 + row * 3;
+                const __nv_bfloat16 zero = __float2bfloat16(0.f);
+                wb[k][h][t] = row >= 9 ? 0u : (s & 1) ? pack_bf16(src[2], zero) : pack_bf16(src[0], src[1]);
+            }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) bias[t][e] = b ? b[channel(t, 2 * q + e)] : 0.f;
+    }
+    // stages slice z: word j of copy 0 = (v[2j], v[2j+1]), of copy 1 = (v[2j+1], v[2j+2]), v[0] at x0 - 1
+    auto stage = [&](int z) {
+        const bool zin = z >= 0 && z < D;
+        uint32_t(*dst)[kInPitch] = ring[(z + 3) % 3];
+        for (int e = tid; e < (kInY + 2) * kInWords; e += 256) {
+            const int r = e / kInWords, j = e - r * kInWords, gy = y0 + r - 1;
+            __nv_bfloat16 v[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int gx = x0 - 1 + 2 * j + k;
+                const bool ok = zin && gy >= 0 && gy < H && gx >= 0 && gx < W;
+                v[k] = __float2bfloat16(ok ? __ldg(vol + ((long)z * H + gy) * W + gx) : 0.f);
+            }
+            dst[r][j] = pack_bf16(v[0], v[1]);
+            dst[r][kInWords + j] = pack_bf16(v[1], v[2]);
         }
+    };
+    stage(z0 - 1);
+    stage(z0);
+    for (int z = z0; z < zend; ++z) {
+        stage(z + 1);
+        __syncthreads();
+        const int gy = y0 + wid;
+        if (gy < H) {
+            const uint32_t* rows[3][2];   // this thread's K pair slots
+            uint32_t mask[3][2];
 #pragma unroll
-        for (int q = 0; q < COUT / 8; ++q) {
-            float f[8];
+            for (int k = 0; k < 3; ++k)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = relu ? fmaxf(acc[8 * q + j], 0.f) : acc[8 * q + j];
-            reinterpret_cast<uint4*>(y + v * COUT)[q] = f_to_bf8(f);
+                for (int h = 0; h < 2; ++h) {
+                    const int s = 8 * k + 4 * h + q, row = min(s >> 1, 8);
+                    rows[k][h] = &ring[(z + row / 3 + 2) % 3][wid + row % 3][(s & 1) + (g & 1) * kInWords + (g >> 1)];
+                    mask[k][h] = s >= 18 ? 0u : (s & 1) ? 0xffffu : 0xffffffffu;
+                }
+            __nv_bfloat16* o = y + (((long)z * H + gy) * W + x0) * COUT;
+#pragma unroll
+            for (int m = 0; m < kInX / 16; ++m) {
+                if (x0 + 16 * m >= W) break;
+                float c[NT][4];
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    c[t][0] = c[t][2] = bias[t][0];
+                    c[t][1] = c[t][3] = bias[t][1];
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const uint32_t a0 = rows[k][0][8 * m] & mask[k][0], a1 = rows[k][0][8 * m + 4] & mask[k][0];
+                    const uint32_t a2 = rows[k][1][8 * m] & mask[k][1], a3 = rows[k][1][8 * m + 4] & mask[k][1];
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) mma_bf16(c[t], a0, a1, a2, a3, wb[k][0][t], wb[k][1][t]);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int x = 16 * m + g + 8 * h;
+                    if (x0 + x < W) {
+                        uint32_t v[NT];
+#pragma unroll
+                        for (int t = 0; t < NT; ++t) {
+                            const float lo = relu ? fmaxf(c[t][2 * h], 0.f) : c[t][2 * h];
+                            const float hi = relu ? fmaxf(c[t][2 * h + 1], 0.f) : c[t][2 * h + 1];
+                            const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+                            v[t] = *reinterpret_cast<const uint32_t*>(&p);
+                        }
+                        uint32_t* dst = reinterpret_cast<uint32_t*>(o + (long)x * COUT) + NT * q;
+                        if constexpr (NT == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+                        else if constexpr (NT == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(v[0], v[1]);
+                        else dst[0] = v[0];
+                    }
+                }
+            }
         }
+        __syncthreads();   // slice z - 1 is replaced by z + 2
     }
 }
 
-// last convolution: CIN input channels -> 1, rounded to BF16, plus the residual volume (FP32)
+// Last convolution: CIN input channels -> 1, rounded to BF16, plus the residual volume (FP32).  The
+// products run on the warp-level tensor cores with the 27 taps as output columns,
+//     P[v][t] = sum_c x[v][c] w[t][c],   out[v] = b + sum_t P[v + off(t)][t],
+// so that every input voxel is read and multiplied once instead of 27 times.  A block marches a
+// 62 x 8 tile of (x, y) down kOutZ slices: per input slice, P of its 64 x 10 halo tile goes to
+// shared memory as [tap][row][x] (pitch 66: the fragments' stores and the sums' loads are free of
+// bank conflicts), and each thread adds the nine taps of each dz into the three output slices that
+// the input slice touches.  K index 2 q + e of the low half is channel 4 q + e of a 16-channel
+// step, of the high half channel 4 q + 2 + e: a thread's operands are one 8-byte load per voxel.
+// 256^3, 16 channels: 498 us (1358 with 27 x 16 scalar FMAs and as many conversions per voxel); bound
+// by the shared-memory passes over P, 27 words written and read per voxel.
+constexpr int kOutX = 62, kOutY = 8, kOutZ = 32, kOutPitch = 66;
+constexpr size_t kOutSmem = sizeof(float) * 27 * (kOutY + 2) * kOutPitch;
+
 template <int CIN>
 __global__ void __launch_bounds__(256) conv_out_kernel(const __nv_bfloat16* __restrict__ x,
                                                        const __nv_bfloat16* __restrict__ w, float b,
                                                        const float* __restrict__ vol, float* __restrict__ out, int D,
-                                                       int H, int W) {
-    __shared__ float sw[27 * CIN];
-    for (int i = threadIdx.x; i < 27 * CIN; i += blockDim.x) sw[i] = __bfloat162float(w[i]);
-    __syncthreads();
-    const long total = (long)D * H * W;
-    for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < total; v += (long)gridDim.x * blockDim.x) {
-        const int xx = (int)(v % W), yy = (int)((v / W) % H), z = (int)(v / ((long)W * H));
-        float acc = b;
-#pragma unroll 3
-        for (int t = 0; t < 27; ++t) {
-            const int sx = xx + t % 3 - 1, sy = yy + (t / 3) % 3 - 1, sz = z + t / 9 - 1;
-            if (sx < 0 || sx >= W || sy < 0 || sy >= H || sz < 0 || sz >= D) continue;
-            const uint4* src = reinterpret_cast<const uint4*>(x + (((long)sz * H + sy) * W + sx) * CIN);
+                                                       int H, int W, int tx, int ty) {
+    constexpr int KS = (CIN + 15) / 16;        // K steps (8 channels: one step, its high half zero)
+    constexpr int CQ = CIN >= 16 ? 4 : 2;      // channels of a step that a thread holds
+    extern __shared__ float P[];               // [27][kOutY + 2][kOutPitch]
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q = lane & 3;
+    const int bx = (int)(blockIdx.x % (unsigned)tx), bt = (int)(blockIdx.x / (unsigned)tx);
+    const int x0 = bx * kOutX, y0 = bt % ty * kOutY, z0 = bt / ty * kOutZ, zend = min(z0 + kOutZ, D);
+    uint32_t wb[KS][4][2];                     // [step][tap tile][K half]
 #pragma unroll
-            for (int q = 0; q < CIN / 8; ++q) {
-                float f[8];
-                bf8_to_f(__ldg(src + q), f);
+    for (int k = 0; k < KS; ++k)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc = fmaf(sw[t * CIN + 8 * q + j], f[j], acc);
+        for (int t = 0; t < 4; ++t) {
+            const int tap = 8 * t + g;
+            const __nv_bfloat16* src = w + (tap < 27 ? tap : 0) * CIN + 16 * k + CQ * q;
+            wb[k][t][0] = tap < 27 ? pack_bf16(src[0], src[1]) : 0u;
+            wb[k][t][1] = tap < 27 && CQ == 4 ? pack_bf16(src[CQ - 2], src[CQ - 1]) : 0u;
+        }
+    // the thread's two output voxels and their sums for slices s - 1, s, s + 1 (s: input slice)
+    const int ox = tid & 63, oy = tid >> 6;    // rows oy and oy + 4
+    float o0[2] = {0.f, 0.f}, o1[2] = {0.f, 0.f}, o2[2];
+    for (int s = max(z0 - 1, 0); s <= min(zend, D - 1); ++s) {
+        // P of the (kOutY + 2) x 64 halo tile: 40 tiles of 16 voxels over 8 warps
+#pragma unroll
+        for (int i = 0; i < (kOutY + 2) * 4 / 8; ++i) {
+            const int mt = wid + 8 * i, r = mt >> 2, xb = (mt & 3) * 16;
+            const int gy = y0 + r - 1;
+            uint32_t a[KS][2][2];              // [step][row g / g + 8][K half]
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int gx = x0 + xb + g + 8 * h - 1;
+                const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
+                const __nv_bfloat16* src = x + (((long)s * H + (ok ? gy : 0)) * W + (ok ? gx : 0)) * CIN + CQ * q;
+#pragma unroll
+                for (int k = 0; k < KS; ++k) {
+                    if constexpr (CQ == 4) {
+                        const uint2 v = ok ? __ldg(reinterpret_cast<const uint2*>(src + 16 * k)) : make_uint2(0u, 0u);
+                        a[k][h][0] = v.x;
+                        a[k][h][1] = v.y;
+                    } else {
+                        a[k][h][0] = ok ? __ldg(reinterpret_cast<const uint32_t*>(src)) : 0u;
+                        a[k][h][1] = 0u;
+                    }
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int k = 0; k < KS; ++k) mma_bf16(c, a[k][0][0], a[k][1][0], a[k][0][1], a[k][1][1], wb[k][t][0], wb[k][t][1]);
+                float* d = P + ((8 * t + 2 * q) * (kOutY + 2) + r) * kOutPitch + xb + g;
+                if (8 * t + 2 * q < 27) {
+                    d[0] = c[0];
+                    d[8] = c[2];
+                }
+                if (8 * t + 2 * q + 1 < 27) {
+                    d[(kOutY + 2) * kOutPitch] = c[1];
+                    d[(kOutY + 2) * kOutPitch + 8] = c[3];
+                }
             }
         }
-        out[v] = vol[v] + __bfloat162float(__float2bfloat16(acc));
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            o2[h] = 0.f;
+            if (ox < kOutX) {
+                float sum[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+                for (int t = 0; t < 27; ++t)
+                    sum[t / 9] += P[(t * (kOutY + 2) + oy + 4 * h + t / 3 % 3) * kOutPitch + ox + t % 3];
+                o0[h] += sum[2];   // dz = 2: input slice s is z + 1 of output slice s - 1
+                o1[h] += sum[1];
+                o2[h] = sum[0];
+                const int gx = x0 + ox, gy = y0 + oy + 4 * h;
+                auto put = [&](int z, float acc) {
+                    const long i = ((long)z * H + gy) * W + gx;
+                    out[i] = __ldg(vol + i) + __bfloat162float(__float2bfloat16(b + acc));
+                };
+                if (gx < W && gy < H) {
+                    if (s - 1 >= z0) put(s - 1, o0[h]);
+                    if (s == D - 1 && s < zend) put(s, o1[h]);   // no slice above the last
+                }
+            }
+            o0[h] = o1[h];
+            o1[h] = o2[h];
+        }
+        __syncthreads();   // P is rewritten for the next slice
     }
 }
 
@@ -183,13 +354,16 @@ int tigre_unet_conv_in(const float* d_vol, const void* d_w, const float* d_b, vo
                        long Cout, int relu, void* stream) {
     if (!d_vol || !d_w || !d_y || D <= 0 || H <= 0 || W <= 0 || !aligned16(d_y))
         return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_in: bad arguments");
-    const long n = D * H * W;
     cudaStream_t st = (cudaStream_t)stream;
     const __nv_bfloat16* w = (const __nv_bfloat16*)d_w;
     __nv_bfloat16* y = (__nv_bfloat16*)d_y;
-    if (Cout == 8) conv_in_kernel<8><<<grid_for(n), 256, 0, st>>>(d_vol, w, d_b, y, (int)D, (int)H, (int)W, relu);
-    else if (Cout == 16) conv_in_kernel<16><<<grid_for(n), 256, 0, st>>>(d_vol, w, d_b, y, (int)D, (int)H, (int)W, relu);
-    else if (Cout == 32) conv_in_kernel<32><<<grid_for(n), 256, 0, st>>>(d_vol, w, d_b, y, (int)D, (int)H, (int)W, relu);
+    const long tx = (W + kInX - 1) / kInX, ty = (H + kInY - 1) / kInY, blocks = tx * ty * ((D + kInZ - 1) / kInZ);
+    if (blocks > INT_MAX || D > INT_MAX - 64 || H > INT_MAX - 64 || W > INT_MAX - 128)
+        return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_in: volume too large");
+    auto go = [&](auto kern) { kern<<<(unsigned)blocks, 256, 0, st>>>(d_vol, w, d_b, y, (int)D, (int)H, (int)W, (int)tx, (int)ty, relu); };
+    if (Cout == 8) go(conv_in_kernel<8>);
+    else if (Cout == 16) go(conv_in_kernel<16>);
+    else if (Cout == 32) go(conv_in_kernel<32>);
     else return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_in: Cout must be 8, 16 or 32");
     TIGRE_LAUNCHED();
     return TIGRE_SUCCESS;
@@ -199,16 +373,22 @@ int tigre_unet_conv_out(const void* d_x, long Cin, const void* d_w, float b, con
                         long H, long W, void* stream) {
     if (!d_x || !d_w || !d_vol || !d_out || D <= 0 || H <= 0 || W <= 0 || !aligned16(d_x))
         return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_out: bad arguments");
-    const long n = D * H * W;
     cudaStream_t st = (cudaStream_t)stream;
     const __nv_bfloat16* x = (const __nv_bfloat16*)d_x;
     const __nv_bfloat16* w = (const __nv_bfloat16*)d_w;
-    if (Cin == 8) conv_out_kernel<8><<<grid_for(n), 256, 0, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W);
-    else if (Cin == 16) conv_out_kernel<16><<<grid_for(n), 256, 0, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W);
-    else if (Cin == 32) conv_out_kernel<32><<<grid_for(n), 256, 0, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W);
-    else return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_out: Cin must be 8, 16 or 32");
-    TIGRE_LAUNCHED();
-    return TIGRE_SUCCESS;
+    const long tx = (W + kOutX - 1) / kOutX, ty = (H + kOutY - 1) / kOutY, blocks = tx * ty * ((D + kOutZ - 1) / kOutZ);
+    if (blocks > INT_MAX || D > INT_MAX - 64 || H > INT_MAX - 64 || W > INT_MAX - 128)
+        return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_out: volume too large");
+    auto go = [&](auto kern) -> int {
+        TIGRE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOutSmem));
+        kern<<<(unsigned)blocks, 256, kOutSmem, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W, (int)tx, (int)ty);
+        TIGRE_LAUNCHED();
+        return TIGRE_SUCCESS;
+    };
+    if (Cin == 8) return go(conv_out_kernel<8>);
+    if (Cin == 16) return go(conv_out_kernel<16>);
+    if (Cin == 32) return go(conv_out_kernel<32>);
+    return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_out: Cin must be 8, 16 or 32");
 }
 
 }  // extern "C"
