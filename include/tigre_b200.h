@@ -316,6 +316,11 @@ int tigre_conv3d_set_tcgen05(int mode);
 int tigre_conv3d_status(int reset);
 int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void* d_y_bf16, float* d_y_f32, long D,
                      long H, long W, long Cin, long Cout, int relu, void* d_col, void* stream);
+/* y (BF16) = conv of the channel concatenation [xa (Ca), xb (Cb)], each read where it is.
+ * tigre_conv3d_fwd_pair_ok: 1 where this form runs (multiples of 16 channels, forward path 3). */
+int tigre_conv3d_fwd_pair_ok(long D, long H, long W, long Ca, long Cb, long Cout);
+int tigre_conv3d_fwd_pair(const void* d_xa, long Ca, const void* d_xb, long Cb, const void* d_w, const float* d_bias,
+                          void* d_y_bf16, long D, long H, long W, long Cout, int relu, void* d_col, void* stream);
 int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D, long H, long W, long Cin, long Cout,
                           float* d_dcol, void* stream);
 int tigre_conv3d_bwd_weight(const void* d_x, const void* d_dy, float* d_dw, long D, long H, long W, long Cin,
@@ -333,6 +338,7 @@ int tigre_conv3d_relu_grad(const void* d_dy, const void* d_y, void* d_g, float* 
  * channels-last activations with FP32 arithmetic; buffers 16-byte aligned.
  * pool2: y (D/2, H/2, W/2, C) = 2x2x2 mean of x (D, H, W, C); even sizes, C % 8 == 0.
  * up_concat: out (D, H, W, Ca + Cb) = [nearest 2x upsampling of low (D/2, H/2, W/2, Ca), skip].
+ * up2: out (D, H, W, C) = nearest 2x upsampling of low (D/2, H/2, W/2, C).
  * conv_in: the first 3x3x3 convolution, one input channel: y (D, H, W, Cout) BF16 from the FP32
  *   volume rounded to BF16, weights w[Cout][27] BF16, bias FP32 (may be NULL), ReLU if relu;
  *   Cout 8, 16 or 32.
@@ -341,6 +347,7 @@ int tigre_conv3d_relu_grad(const void* d_dy, const void* d_y, void* d_g, float* 
 int tigre_unet_pool2(const void* d_x, void* d_y, long D, long H, long W, long C, void* stream);
 int tigre_unet_up_concat(const void* d_low, long Ca, const void* d_skip, long Cb, void* d_out, long D, long H, long W,
                          void* stream);
+int tigre_unet_up2(const void* d_low, void* d_out, long D, long H, long W, long C, void* stream);
 int tigre_unet_conv_in(const float* d_vol, const void* d_w, const float* d_b, void* d_y, long D, long H, long W,
                        long Cout, int relu, void* stream);
 int tigre_unet_conv_out(const void* d_x, long Cin, const void* d_w, float b, const float* d_vol, float* d_out, long D,

@@ -127,9 +127,13 @@ _SIGS = {
                                       C.c_long, C.c_long, C.c_void_p]),
     "tigre_conv3d_fwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long,
                                    C.c_long, C.c_long, C.c_long, C.c_int, C.c_void_p, C.c_void_p]),
+    "tigre_conv3d_fwd_pair_ok": (C.c_int, [C.c_long] * 6),
+    "tigre_conv3d_fwd_pair": (C.c_int, [C.c_void_p, C.c_long, C.c_void_p, C.c_long, C.c_void_p, C.c_void_p, C.c_void_p,
+                                        C.c_long, C.c_long, C.c_long, C.c_long, C.c_int, C.c_void_p, C.c_void_p]),
     "tigre_conv3d_relu_grad_work": (C.c_longlong, [C.c_long, C.c_long]),
     "tigre_conv3d_relu_grad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long, C.c_int,
                                          C.c_void_p, C.c_void_p]),
+    "tigre_unet_up2": (C.c_int, [C.c_void_p, C.c_void_p, C.c_long, C.c_long, C.c_long, C.c_long, C.c_void_p]),
     "tigre_conv3d_bwd_data": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long, C.c_long, C.c_long,
                                         C.c_long, C.c_void_p, C.c_void_p]),
     "tigre_conv3d_bwd_weight": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long, C.c_long, C.c_long,

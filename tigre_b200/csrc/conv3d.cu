@@ -558,7 +558,7 @@ int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void
     int* status = conv_status_word();
     if (tc_mode == 3 && ((uintptr_t)d_x & 15) == 0 && ((uintptr_t)d_col & 15) == 0 &&
         27L * Cin * Cout <= tigre_conv3d_col_elems(D, H, W, Cin) && conv_tc_halo_supported(D, H, W, Cin, Cout))
-        return launch_conv_tc_halo((const __nv_bfloat16*)d_x, (const __nv_bfloat16*)d_w, d_bias,
+        return launch_conv_tc_halo((const __nv_bfloat16*)d_x, nullptr, 0, (const __nv_bfloat16*)d_w, d_bias,
                                    (__nv_bfloat16*)d_y_bf16, d_y_f32, D, H, W, Cin, Cout, relu, 0,
                                    (__nv_bfloat16*)d_col, status, st);
     if (tc_mode == 3) tc_mode = 2;
@@ -607,6 +607,24 @@ int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void
     return TIGRE_SUCCESS;
 }
 
+// y = conv([xa, xb]) for an input that lies in two buffers: the halo-tile kernel reads each where it
+// is; 0 where it cannot (the caller then concatenates).
+int tigre_conv3d_fwd_pair_ok(long D, long H, long W, long Ca, long Cb, long Cout) {
+    return D > 0 && H > 0 && W > 0 && Ca > 0 && Cb > 0 && Ca % 16 == 0 && Cb % 16 == 0 && g_conv_tcgen05.load() == 3 &&
+           Cout <= D * H * W && conv_tc_halo_supported(D, H, W, Ca + Cb, Cout);
+}
+
+int tigre_conv3d_fwd_pair(const void* d_xa, long Ca, const void* d_xb, long Cb, const void* d_w, const float* d_bias,
+                          void* d_y_bf16, long D, long H, long W, long Cout, int relu, void* d_col, void* stream) {
+    TIGRE_NVTX("tigre_conv3d_fwd_pair");
+    if (!d_xa || !d_xb || !d_w || !d_y_bf16 || !d_col) return fail(TIGRE_ERR_BAD_ASSERT, "bad conv3d arguments");
+    if (!tigre_conv3d_fwd_pair_ok(D, H, W, Ca, Cb, Cout) || (((uintptr_t)d_xa | (uintptr_t)d_xb | (uintptr_t)d_col) & 15))
+        return fail(TIGRE_ERR_BAD_ASSERT, "conv3d of a pair: channels in multiples of 16, 16-byte aligned buffers");
+    return launch_conv_tc_halo((const __nv_bfloat16*)d_xa, (const __nv_bfloat16*)d_xb, Cb, (const __nv_bfloat16*)d_w, d_bias,
+                               (__nv_bfloat16*)d_y_bf16, nullptr, D, H, W, Ca + Cb, Cout, relu, 0, (__nv_bfloat16*)d_col,
+                               conv_status_word(), (cudaStream_t)stream);
+}
+
 // dx (FP32, channels-last) from dy (BF16, M x Cout) and w; d_dcol: M * 27*Cin floats of scratch.
 int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D, long H, long W, long Cin, long Cout,
                           float* d_dcol, void* stream) {
@@ -619,7 +637,7 @@ int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D
         Cout <= 2 * M && conv_tc_halo_supported(D, H, W, Cout, Cin)) {   // d_dcol holds the arranged weights
         // the data gradient is the convolution of dy with the tap-flipped, channel-transposed
         // weights: the halo kernel, FP32 output, no im2col (d_dcol holds the arranged weights)
-        return launch_conv_tc_halo((const __nv_bfloat16*)d_dy, (const __nv_bfloat16*)d_w, nullptr, nullptr, d_dx, D,
+        return launch_conv_tc_halo((const __nv_bfloat16*)d_dy, nullptr, 0, (const __nv_bfloat16*)d_w, nullptr, nullptr, d_dx, D,
                                    H, W, Cin, Cout, 0, 1, (__nv_bfloat16*)d_dcol, conv_status_word(), st);
     }
     dim3 grid((unsigned)((M + kBM - 1) / kBM), (unsigned)((K + kBN - 1) / kBN), 1);

@@ -72,11 +72,13 @@ struct ConvTcArgs {
     int* status;
     int D, H, W, Cin, Cout, relu;
     int zt, stages, nchunks;
+    int chunks_a;              // the first chunks come from the first tensor map, the others from the second
     uint32_t tile_bytes, w_bytes, stage_bytes, tmem_cols;
 };
 
 template <int MAXS>
-__global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_constant__ CUtensorMap xmap, ConvTcArgs p) {
+__global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_constant__ CUtensorMap xmap,
+                                                              const __grid_constant__ CUtensorMap xmap_b, ConvTcArgs p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long full_bar[MAXS], empty_bar[MAXS], done_bar;
     __shared__ uint32_t tmem_slot;
@@ -121,10 +123,12 @@ __global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_const
             const uint32_t fb = su32(&full_bar[s]);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(p.tile_bytes + p.w_bytes)
                          : "memory");
+            const bool in_a = c < p.chunks_a;
+            const unsigned long long map = in_a ? (unsigned long long)&xmap : (unsigned long long)&xmap_b;
             asm volatile(
                 "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], "
                 "[%7];" ::"r"(st),
-                "l"((unsigned long long)&xmap), "r"(0), "r"(x0 - 1), "r"(c * (kCC / 8)), "r"(y0 - 1), "r"(z0 - 1), "r"(fb)
+                "l"(map), "r"(0), "r"(x0 - 1), "r"((in_a ? c : c - p.chunks_a) * (kCC / 8)), "r"(y0 - 1), "r"(z0 - 1), "r"(fb)
                 : "memory");
             const __nv_bfloat16* src = p.wk + (size_t)c * (p.w_bytes / 2);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -328,7 +332,9 @@ bool conv_tc_halo_supported(long D, long H, long W, long Cin, long Cout) {
 // convolution instead: x is then the gradient of the output (Cout channels), y the gradient of
 // the input (Cin channels), with the weights flipped in the taps and transposed in the channels
 // (arrange_weights_kernel).  wk_scratch: 27 Cin Cout BF16 elements, 16-byte aligned.
-int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias, __nv_bfloat16* yb,
+// xb != nullptr (not with flip): the input is the channel concatenation of x (Cin - Cb channels)
+// and xb (Cb), each a multiple of 16, read from where they are.
+int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* xb, long Cb, const __nv_bfloat16* w, const float* bias, __nv_bfloat16* yb,
                         float* yf, long D, long H, long W, long Cin, long Cout, int relu, int flip,
                         __nv_bfloat16* wk_scratch, int* status, cudaStream_t st) {
     // K (input channels of this convolution) and N (its output channels)
@@ -341,16 +347,21 @@ int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* w, const fl
     arrange_weights_kernel<<<(int)std::min<long>((total + 255) / 256, 148L * 16), 256, 0, st>>>(w, wk_scratch, (int)Cin,
                                                                                                 (int)Cout, flip);
     TIGRE_LAUNCHED();
-    // x as a 5-D tensor, innermost first: 8 channels, x, chunks of 8 channels, y, z
-    CUtensorMap tm;
-    cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)(K / 8), (cuuint64_t)H, (cuuint64_t)D};
-    cuuint64_t strides[4] = {(cuuint64_t)(K * 2), 16, (cuuint64_t)(W * K * 2), (cuuint64_t)(H * W * K * 2)};
-    cuuint32_t box[5] = {8, (cuuint32_t)kHx, (cuuint32_t)(kCC / 8), (cuuint32_t)kHy, (cuuint32_t)(zt + 2)};
-    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    CUresult r = encode_tiled()(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16*>(x), dims, strides,
-                                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(TIGRE_ERR_CUDA, "cuTensorMapEncodeTiled (conv halo tile) failed");
+    // the inputs as 5-D tensors, innermost first: 8 channels, x, chunks of 8 channels, y, z
+    CUtensorMap maps[2];
+    const __nv_bfloat16* src[2] = {x, xb ? xb : x};
+    const long chan[2] = {xb ? K - Cb : K, xb ? Cb : K};
+    for (int i = 0; i < 2; ++i) {
+        const cuuint64_t C = (cuuint64_t)chan[i];
+        cuuint64_t dims[5] = {8, (cuuint64_t)W, C / 8, (cuuint64_t)H, (cuuint64_t)D};
+        cuuint64_t strides[4] = {C * 2, 16, (cuuint64_t)W * C * 2, (cuuint64_t)(H * W) * C * 2};
+        cuuint32_t box[5] = {8, (cuuint32_t)kHx, (cuuint32_t)(kCC / 8), (cuuint32_t)kHy, (cuuint32_t)(zt + 2)};
+        cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+        CUresult r = encode_tiled()(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16*>(src[i]), dims,
+                                    strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(TIGRE_ERR_CUDA, "cuTensorMapEncodeTiled (conv halo tile) failed");
+    }
     ConvTcArgs a{};
     a.wk = wk_scratch;
     a.bias = bias;
@@ -361,6 +372,7 @@ int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* w, const fl
     a.zt = zt;
     a.stages = stages;
     a.nchunks = (int)(K / kCC);
+    a.chunks_a = (int)(chan[0] / kCC);
     a.tile_bytes = tb;
     a.w_bytes = wb;
     a.stage_bytes = (tb + wb + 1023u) & ~1023u;
@@ -375,7 +387,7 @@ int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* w, const fl
     const size_t smem = std::max(need, floor_smem);
     TIGRE_CUDA(cudaFuncSetAttribute(conv_tc_halo_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long ntiles = ((W + kTx - 1) / kTx) * ((H + kTy - 1) / kTy) * ((D + zt - 1) / zt);
-    conv_tc_halo_kernel<3><<<(unsigned)ntiles, 128, smem, st>>>(tm, a);
+    conv_tc_halo_kernel<3><<<(unsigned)ntiles, 128, smem, st>>>(maps[0], maps[1], a);
     TIGRE_LAUNCHED();
     return TIGRE_SUCCESS;
 }

@@ -82,6 +82,25 @@ __global__ void up_concat_kernel(const uint4* __restrict__ low, int Ca8, const u
     }
 }
 
+// out[z][y][x] = low[z/2][y/2][x/2]: one thread per 16 bytes of low, eight stores
+__global__ void __launch_bounds__(256) up2_kernel(const uint4* __restrict__ low, uint4* __restrict__ out, int d, int h, int w,
+                                                  int C8) {
+    const long row = (long)w * C8, total = (long)d * h * row;
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
+        const long v = e / C8;
+        const int c = (int)(e - v * C8), x = (int)(v % w);
+        const long zy = v / w;
+        const int y = (int)(zy % h), z = (int)(zy / h);
+        const uint4 val = __ldg(low + e);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            uint4* o = out + (((2L * z + (k >> 1)) * (2 * h) + 2 * y + (k & 1)) * (2L * w) + 2 * x) * C8 + c;
+            o[0] = val;
+            o[C8] = val;
+        }
+    }
+}
+
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
     asm volatile(
@@ -346,6 +365,17 @@ int tigre_unet_up_concat(const void* d_low, long Ca, const void* d_skip, long Cb
     up_concat_kernel<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const uint4*)d_low, (int)(Ca / 8),
                                                                   (const uint4*)d_skip, (int)(Cb / 8), (uint4*)d_out,
                                                                   (int)D, (int)H, (int)W);
+    TIGRE_LAUNCHED();
+    return TIGRE_SUCCESS;
+}
+
+int tigre_unet_up2(const void* d_low, void* d_out, long D, long H, long W, long C, void* stream) {
+    if (!d_low || !d_out || D % 2 || H % 2 || W % 2 || D <= 0 || H <= 0 || W <= 0 || C % 8 || C <= 0 || !aligned16(d_low) ||
+        !aligned16(d_out))
+        return fail(TIGRE_ERR_BAD_ASSERT, "unet up2: even sizes, channels % 8 == 0, 16-byte aligned buffers");
+    const long n = (D / 2) * (H / 2) * (W / 2) * (C / 8);
+    up2_kernel<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const uint4*)d_low, (uint4*)d_out, (int)(D / 2), (int)(H / 2),
+                                                            (int)(W / 2), (int)(C / 8));
     TIGRE_LAUNCHED();
     return TIGRE_SUCCESS;
 }

@@ -249,6 +249,17 @@ def _make_unet_class():
                 x = conv(conv(pooled, self.enc[i][0]), self.enc[i][1])
             for (ca, cb), s in zip(self.dec, reversed(skips)):
                 d, h, w, cs = s.shape
+                cx, co = x.shape[-1], ca.w.shape[0]
+                if L.tigre_conv3d_fwd_pair_ok(d, h, w, cx, cs, co):
+                    # the convolution reads the upsampled level and the skip connection where they are
+                    up = T.empty((d, h, w, cx), dtype=T.bfloat16, device=x.device)
+                    N.check(L.tigre_unet_up2(p(x), p(up), d, h, w, cx, st), "tigre_unet_up2")
+                    y = T.empty((d, h, w, co), dtype=T.bfloat16, device=x.device)
+                    col = _SCRATCH.get(27 * (cx + cs) * co, "col", x.device)
+                    N.check(L.tigre_conv3d_fwd_pair(p(up), cx, p(s), cs, p(self._wbf(ca)), p(ca.b), p(y), d, h, w, co,
+                                                    1 if ca.relu else 0, p(col), st), "tigre_conv3d_fwd_pair")
+                    x = conv(y, cb)
+                    continue
                 cat = T.empty((d, h, w, x.shape[-1] + cs), dtype=T.bfloat16, device=x.device)
                 N.check(L.tigre_unet_up_concat(p(x), x.shape[-1], p(s), cs, p(cat), d, h, w, st),
                         "tigre_unet_up_concat")
