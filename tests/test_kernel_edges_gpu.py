@@ -64,6 +64,28 @@ def test_backprojection_with_shared_views(shape, views, kind):
     assert plan.status() == 0
 
 
+# ------------------------------------------------------------------- Siddon: z-fast working copy --
+@pytest.mark.parametrize("shape,det", [
+    ((64, 64, 64), (33, 40)),      # four elements per access on both sides
+    ((63, 5, 62), (20, 21)),       # rows of the volume no multiple of four
+    ((7, 9, 68), (256, 12)),       # rows in fours, runs of the copy shorter than a tile
+    ((130, 66, 132), (513, 9)),    # one past a tile in every axis
+])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16"])
+@pytest.mark.parametrize("shift", [0, 1])   # the volume starts on an odd element of a larger buffer
+def test_siddon_over_the_zfast_copy(shape, det, dtype, shift):
+    import torch
+    from tigre_b200 import projectors as P
+    geo = _geo(shape, det, 160.0 / max(det), offsets=True)
+    ang = G.angles(5)
+    dt = getattr(torch, dtype)
+    n = int(np.prod(shape))
+    flat = torch.from_numpy(np.random.default_rng(n).random(n + shift, dtype=np.float32)).cuda().to(dt)
+    vol = flat[shift:].view(shape)
+    ref = O.ax(vol.float().cpu().numpy(), geo, ang, "Siddon")
+    _close(P.ax(vol, _plan(geo, ang), "Siddon", out_dtype=torch.float32).cpu().numpy(), ref)
+
+
 # --------------------------------------------------------- backprojection: tilted frames --
 @pytest.mark.parametrize("shape", [(64, 16, 16), (65, 17, 18), (3, 30, 5), (130, 20, 33)])
 @pytest.mark.parametrize("kind", ["FDK", "matched"])
