@@ -86,6 +86,43 @@ def test_siddon_over_the_zfast_copy(shape, det, dtype, shift):
     _close(P.ax(vol, _plan(geo, ang), "Siddon", out_dtype=torch.float32).cpu().numpy(), ref)
 
 
+# Cells are listed 32 at a time: lists that end in a full one, start a new one for a single cell, and
+# crossings of both axes at one point (45 degrees); 8, 4 and 2 rows per thread with remainders.
+@pytest.mark.parametrize("xy", [(1, 1), (16, 16), (17, 16), (33, 31), (32, 33), (96, 97)])
+@pytest.mark.parametrize("nv", [3, 65, 200, 257])
+@pytest.mark.parametrize("mode", ["cone", "parallel"])
+def test_siddon_cell_lists(xy, nv, mode):
+    import torch
+    from tigre_b200 import projectors as P
+    shape = (24, xy[1], xy[0])
+    geo = _geo(shape, (nv, 14), 40.0 / nv, offsets=True, mode=mode)
+    geo.dDetector = np.array((40.0 / nv, 1.7 * max(xy) / 14))
+    geo.sDetector = geo.nDetector * geo.dDetector
+    ang = np.array([0.0, 0.25, 0.5, 0.31, 0.75, 1.25, 1.5, 1.9]) * np.pi
+    vol = np.random.default_rng(nv).random(shape, dtype=np.float32)
+    got = P.ax(torch.from_numpy(vol).cuda(), _plan(geo, ang.astype(np.float32)), "Siddon")
+    _close(got.cpu().numpy(), O.ax(vol, geo, ang.astype(np.float32), "Siddon"))
+
+
+@pytest.mark.parametrize("nv", [24, 100, 256])
+def test_siddon_copy_beyond_one_window(nv):
+    """A working copy larger than 4 GB, so that its addresses differ in their high words, against the
+    stepped column kernel; the steepest rows leave the volume through its faces."""
+    import torch
+    from tigre_b200 import _native as N, projectors as P
+    shape = (48, 4500, 4400)
+    geo = _geo(shape, (nv, 6), 100.0 / nv, dso=20000.0, dsd=30000.0, offsets=True)
+    geo.dDetector = np.array((100.0 / nv, 1000.0))
+    geo.sDetector = geo.nDetector * geo.dDetector
+    ang = np.linspace(0.0, 2.0, 4, dtype=np.float32)
+    vol = torch.rand(shape, device="cuda", generator=torch.Generator("cuda").manual_seed(nv))
+    got = P.ax(vol, _plan(geo, ang), "Siddon")
+    with N.option(N.OPT_SIDDON_KERNEL, 1):
+        ref = P.ax(vol, _plan(geo, ang), "Siddon")
+    assert float(ref.max()) > 100.0
+    _close(got.cpu().numpy(), ref.cpu().numpy(), 2 * TOL)
+
+
 # --------------------------------------------------------- backprojection: tilted frames --
 @pytest.mark.parametrize("shape", [(64, 16, 16), (65, 17, 18), (3, 30, 5), (130, 20, 33)])
 @pytest.mark.parametrize("kind", ["FDK", "matched"])

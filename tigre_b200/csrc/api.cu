@@ -165,7 +165,7 @@ int ax_prepare(TigrePlan* plan, const void* d_vol, int vdt, int projector, int a
 
 int ax_launch(TigrePlan* plan, const AxWork& w, void* d_proj, int pdt, int a0, int a1, cudaStream_t st) {
     switch (w.mode) {
-        case AxWork::CELLS: return launch_siddon_cells(plan, w.vx, w.vdt, d_proj, pdt, a0, a1, st);
+        case AxWork::CELLS: return launch_siddon_cells(plan, (const float*)w.vx, d_proj, pdt, a0, a1, st);
         case AxWork::COLUMNS: return launch_siddon_columns(plan, w.vx, w.vdt, d_proj, pdt, a0, a1, st);
         case AxWork::GENERAL: return launch_siddon(plan, w.vx, w.vy, w.vdt, d_proj, pdt, a0, a1, st);
         case AxWork::INTERP_TEX: return launch_interp_tex(plan, w.tex, d_proj, pdt, a0, a1, st);

@@ -174,8 +174,7 @@ int launch_siddon(TigrePlan* p, const void* vol_x, const void* vol_y, int vdt, v
                   cudaStream_t st);
 int launch_siddon_count(TigrePlan* p, int a0, int a1, unsigned long long* d_total, cudaStream_t st);
 int launch_interp_count(TigrePlan* p, int a0, int a1, unsigned long long* d_total, cudaStream_t st);
-int launch_siddon_cells(TigrePlan* p, const void* vol_z, int vdt, void* proj, int pdt, int a0, int a1,
-                        cudaStream_t st);
+int launch_siddon_cells(TigrePlan* p, const float* vol_z, void* proj, int pdt, int a0, int a1, cudaStream_t st);
 int launch_siddon_columns(TigrePlan* p, const void* vol_z, int vdt, void* proj, int pdt, int a0, int a1,
                           cudaStream_t st);
 int launch_interp(TigrePlan* p, const void* vol_x, const void* vol_y, const void* quad_x, const void* quad_y, int vdt,
