@@ -89,16 +89,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
     return false;
 }
 
-template <typename TP> __device__ __forceinline__ float lds(uint32_t a);
-template <> __device__ __forceinline__ float lds<float>(uint32_t a) {
+__device__ __forceinline__ float lds(uint32_t a) {
     float v;
     asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
     return v;
-}
-template <> __device__ __forceinline__ float lds<__nv_bfloat16>(uint32_t a) {
-    unsigned short v;
-    asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-    return __uint_as_float(((unsigned)v) << 16);
 }
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
@@ -130,9 +124,8 @@ __device__ __forceinline__ void project_texel(const FrameBPK& F, float x, float 
 // info[] and issues the TMA load (or a plain arrive when the box does not fit), unless
 // `stopped` (lane 0's own wait for an earlier view expired: the buffer may still be awaiting
 // that copy, so its barrier must not be re-armed).
-template <typename TP>
 __device__ __forceinline__ void plan_patch(const BPKArgs& p, const CUtensorMap* tmap, int la, int x0, int y0, int z0,
-                                           TP* dst, uint32_t bar, int* info, bool stopped) {
+                                           float* dst, uint32_t bar, int* info, bool stopped) {
     const int lane = threadIdx.x & 31;
     const FrameBPK& F = p.frames[p.a0 + la];
     float ub = 0.f, vb = 0.f;
@@ -153,7 +146,7 @@ __device__ __forceinline__ void plan_patch(const BPKArgs& p, const CUtensorMap* 
     }
     if (lane == 0) {
         if (stopped) return;
-        constexpr int ALIGN = 16 / (int)sizeof(TP);   // TMA: x * sizeof(T) multiple of 16 bytes
+        constexpr int ALIGN = 4;   // TMA: x * sizeof(float) a multiple of 16 bytes
         bool fits = isfinite(umin) && isfinite(umax) && isfinite(vmin) && isfinite(vmax) &&
                     fabsf(umin) < 1e7f && fabsf(vmin) < 1e7f;
         int u0 = 0, v0 = 0;
@@ -171,7 +164,7 @@ __device__ __forceinline__ void plan_patch(const BPKArgs& p, const CUtensorMap* 
             // failure-detection test: neither a copy nor an arrival, so the wait for this view
             // runs out with nothing in flight
         } else if (fits) {
-            const uint32_t bytes = (uint32_t)(p.BU * p.BV * sizeof(TP));
+            const uint32_t bytes = (uint32_t)(p.BU * p.BV * sizeof(float));
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
             asm volatile(
                 "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
@@ -184,20 +177,19 @@ __device__ __forceinline__ void plan_patch(const BPKArgs& p, const CUtensorMap* 
     }
 }
 
-template <typename TP>
-__device__ __forceinline__ float global_sample(const BPKArgs& p, const TP* P, float ub, float vb) {
+__device__ __forceinline__ float global_sample(const BPKArgs& p, const float* P, float ub, float vb) {
     const float fx = floorf(ub), fy = floorf(vb);
     const float au = ub - fx, av = vb - fy;
     const int iu = (int)fmaxf(fminf(fx, 1e8f), -1e8f), iv = (int)fmaxf(fminf(fy, 1e8f), -1e8f);
     auto at = [&](int u, int v) -> float {
-        return (u >= 0 && u < p.nU && v >= 0 && v < p.nV) ? to_f32<TP>(P[(long)v * p.pitch + u]) : 0.f;
+        return (u >= 0 && u < p.nU && v >= 0 && v < p.nV) ? P[(long)v * p.pitch + u] : 0.f;
     };
     const float a0 = fmaf(au, at(iu + 1, iv) - at(iu, iv), at(iu, iv));
     const float a1 = fmaf(au, at(iu + 1, iv + 1) - at(iu, iv + 1), at(iu, iv + 1));
     return fmaf(av, a1 - a0, a0);
 }
 
-template <typename TP, typename TV, bool MATCHED, bool AXIAL, bool SPLIT>
+template <typename TV, bool MATCHED, bool AXIAL, bool SPLIT>
 __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, BPKArgs p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[2];
@@ -209,11 +201,11 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
     const int nviews = (SPLIT ? (int)((long)p.na * (rank + 1) / p.nsplit) : p.na) - lb;
     // TMA destinations: 128-byte aligned, each buffer rounded up to 128 bytes
     const uint32_t base_off = (128u - (smem_u32(smem_raw) & 127u)) & 127u;
-    const size_t buf_bytes = ((size_t)p.BU * p.BV * sizeof(TP) + 127) / 128 * 128;
-    TP* buf0 = reinterpret_cast<TP*>(smem_raw + base_off);
-    TP* buf1 = reinterpret_cast<TP*>(smem_raw + base_off + buf_bytes);
+    const size_t buf_bytes = ((size_t)p.BU * p.BV * sizeof(float) + 127) / 128 * 128;
+    float* buf0 = reinterpret_cast<float*>(smem_raw + base_off);
+    float* buf1 = reinterpret_cast<float*>(smem_raw + base_off + buf_bytes);
     const uint32_t buf0_u32 = smem_u32(buf0), buf1_u32 = smem_u32(buf1);
-    const uint32_t rowb = (uint32_t)(p.BU * sizeof(TP));
+    const uint32_t rowb = (uint32_t)(p.BU * sizeof(float));
     const int tid = threadIdx.x;
     // each warp covers an 8 x 4 patch of columns: at every view angle its 32 samples of one
     // slice fall on a compact set of detector texels (few shared-memory wavefronts)
@@ -232,13 +224,13 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
     }
     __syncthreads();
     if (tid < 32) {
-        plan_patch<TP>(p, &tmap, lb, x0, y0, z0, buf0, bar0, info[0], false);
-        if (nviews > 1) plan_patch<TP>(p, &tmap, lb + 1, x0, y0, z0, buf1, bar1, info[1], false);
+        plan_patch(p, &tmap, lb, x0, y0, z0, buf0, bar0, info[0], false);
+        if (nviews > 1) plan_patch(p, &tmap, lb + 1, x0, y0, z0, buf1, bar1, info[1], false);
     }
     float acc[VZ];
 #pragma unroll
     for (int k = 0; k < VZ; ++k) acc[k] = 0.f;
-    const TP* Pg = (const TP*)p.proj;
+    const float* Pg = (const float*)p.proj;
     const float pumax = (float)(p.BU - 2), pvmax = (float)(p.BV - 2);
     int failed_at = -1;   // first view (of this block's) whose wait expired in this thread
     for (int i = 0; i < nviews; ++i) {
@@ -247,7 +239,7 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
         const uint32_t bar = s ? bar1 : bar0;
         // after one expired wait this thread waits no more (its sums are not written)
         if (failed_at < 0 && !mbar_wait(bar, (uint32_t)((i >> 1) & 1))) failed_at = i;
-        const TP* patch = s ? buf1 : buf0;
+        const float* patch = s ? buf1 : buf0;
         const uint32_t patch_u32 = s ? buf1_u32 : buf0_u32;
         const int u0 = info[s][0], v0 = info[s][1], fits = info[s][2];
         if (active) {
@@ -280,7 +272,7 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
                     const int iu = (int)pu;
                     const float2 fu2 = f2(pu - (float)iu);
                     const float pv0 = vt0 - 0.5f - (float)v0;
-                    constexpr uint32_t ES = (uint32_t)sizeof(TP);
+                    constexpr uint32_t ES = (uint32_t)sizeof(float);
                     const uint32_t colb = patch_u32 + (uint32_t)iu * ES;
                     const float2 vstep2 = f2(vstep);
                     const float2 pv02 = f2(pv0);
@@ -338,9 +330,9 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
                             const float2 fv = __ffma2_rn(__fadd2_rn(t, f2(-12582912.0f)), f2(-1.f), pv);
                             const uint32_t aa = (uint32_t)__float_as_int(t.x) * rowb + colb_m;
                             const uint32_t ab = (uint32_t)__float_as_int(t.y) * rowb + colb_m;
-                            const float2 r0 = f2(lds<TP>(aa), lds<TP>(ab)), r0r = f2(lds<TP>(aa + ES), lds<TP>(ab + ES));
-                            const float2 r1 = f2(lds<TP>(aa + rowb), lds<TP>(ab + rowb));
-                            const float2 r1r = f2(lds<TP>(aa + rowb + ES), lds<TP>(ab + rowb + ES));
+                            const float2 r0 = f2(lds(aa), lds(ab)), r0r = f2(lds(aa + ES), lds(ab + ES));
+                            const float2 r1 = f2(lds(aa + rowb), lds(ab + rowb));
+                            const float2 r1r = f2(lds(aa + rowb + ES), lds(ab + rowb + ES));
                             const float2 smp = lerp2(lerp2(r0, r0r, fu2), lerp2(r1, r1r, fu2), fv);
                             float2 w = w2;
                             if (MATCHED) {
@@ -359,7 +351,7 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
 #pragma unroll
                     for (int k = 0; k < VZ; ++k) {
                         const float vtex = fmaf((float)k, vstep, vt0);
-                        const float smp = global_sample<TP>(p, Pg + (long)la * p.pitch * p.nV, u - 0.5f, vtex - 0.5f);
+                        const float smp = global_sample(p, Pg + (long)la * p.pitch * p.nV, u - 0.5f, vtex - 0.5f);
                         float w = wcol;
                         if (MATCHED) {
                             const float dz = fmaf(vtex, F.ddv, F.dzc);
@@ -382,7 +374,7 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
                 const float dzx = (float)F.dz[0], dzy = (float)F.dz[1], dzz = (float)F.dz[2];
                 if (fits) {
                     const float cup = F.cu - 0.5f - (float)u0, cvp = F.cv - 0.5f - (float)v0;   // patch coordinates
-                    constexpr uint32_t ES = (uint32_t)sizeof(TP);
+                    constexpr uint32_t ES = (uint32_t)sizeof(float);
                     const uint32_t base = patch_u32 - 0x4B400000u * rowb - 0x4B400000u * ES;
                     const float cw = 0.5f + (float)u0, cz = 0.5f + (float)v0;
                     const float day0 = fmaf(cw, F.ddu, F.du0), dz0 = fmaf(cz, F.ddv, F.dzc);
@@ -419,9 +411,9 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
                             const float2 fv = __ffma2_rn(__fadd2_rn(tv, f2(-12582912.0f)), f2(-1.f), pv);
                             const uint32_t aa = (uint32_t)__float_as_int(tv.x) * rowb + ((uint32_t)__float_as_int(tu.x) * ES + base);
                             const uint32_t ab = (uint32_t)__float_as_int(tv.y) * rowb + ((uint32_t)__float_as_int(tu.y) * ES + base);
-                            const float2 r0 = f2(lds<TP>(aa), lds<TP>(ab)), r0r = f2(lds<TP>(aa + ES), lds<TP>(ab + ES));
-                            const float2 r1 = f2(lds<TP>(aa + rowb), lds<TP>(ab + rowb));
-                            const float2 r1r = f2(lds<TP>(aa + rowb + ES), lds<TP>(ab + rowb + ES));
+                            const float2 r0 = f2(lds(aa), lds(ab)), r0r = f2(lds(aa + ES), lds(ab + ES));
+                            const float2 r1 = f2(lds(aa + rowb), lds(ab + rowb));
+                            const float2 r1r = f2(lds(aa + rowb + ES), lds(ab + rowb + ES));
                             const float2 smp = lerp2(lerp2(r0, r0r, fu), lerp2(r1, r1r, fu), fv);
                             float2 w = f2(wcol);
                             if (MATCHED) {
@@ -447,7 +439,7 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
                         const float ex = fmaf(kf, dzx, vx), ey = fmaf(kf, dzy, vy), ez = fmaf(kf, dzz, vz);
                         const float t = F.tnum / ex;
                         const float u = fmaf(ey, t, F.cu), vtex = fmaf(ez, t, F.cv);
-                        const float smp = global_sample<TP>(p, Pg + (long)la * p.pitch * p.nV, u - 0.5f, vtex - 0.5f);
+                        const float smp = global_sample(p, Pg + (long)la * p.pitch * p.nV, u - 0.5f, vtex - 0.5f);
                         float w = wcol;
                         if (MATCHED) {
                             const float day = fmaf(u, F.ddu, F.du0);
@@ -464,7 +456,7 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
             }
         }
         __syncthreads();   // everyone is done with buffer s
-        if (tid < 32 && i + 2 < nviews) plan_patch<TP>(p, &tmap, la + 2, x0, y0, z0, s ? buf1 : buf0, bar, info[s], failed_at >= 0);
+        if (tid < 32 && i + 2 < nviews) plan_patch(p, &tmap, la + 2, x0, y0, z0, s ? buf1 : buf0, bar, info[s], failed_at >= 0);
     }
     if (tid == 0 && failed_at >= 0) {
         // thread 0 issued nothing after its failed view: the copies of that view and the next
@@ -564,11 +556,11 @@ int bp_splits(long blocks, int na) {
     return best;
 }
 
-template <typename TP, typename TV>
+template <typename TV>
 int launch_typed(const CUtensorMap& tm, BPKArgs a, bool matched, bool axial, cudaStream_t st) {
     dim3 grid((a.nX + TXY - 1) / TXY, (a.nY + TXY - 1) / TXY, (a.nZ + VZ - 1) / VZ);
     a.nsplit = bp_splits((long)grid.x * grid.y * grid.z, a.na);
-    size_t smem = 2 * (((size_t)a.BU * a.BV * sizeof(TP) + 127) / 128 * 128) + 128;
+    size_t smem = 2 * (((size_t)a.BU * a.BV * sizeof(float) + 127) / 128 * 128) + 128;
     auto go = [&](auto kern) -> int {
         TIGRE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kern<<<grid, TXY * TXY, smem, st>>>(tm, a);
@@ -594,11 +586,11 @@ int launch_typed(const CUtensorMap& tm, BPKArgs a, bool matched, bool axial, cud
         return TIGRE_SUCCESS;
     };
     if (a.nsplit > 1) {
-        if (matched) return axial ? go_split(bp_tma_kernel<TP, TV, true, true, true>) : go_split(bp_tma_kernel<TP, TV, true, false, true>);
-        return axial ? go_split(bp_tma_kernel<TP, TV, false, true, true>) : go_split(bp_tma_kernel<TP, TV, false, false, true>);
+        if (matched) return axial ? go_split(bp_tma_kernel<TV, true, true, true>) : go_split(bp_tma_kernel<TV, true, false, true>);
+        return axial ? go_split(bp_tma_kernel<TV, false, true, true>) : go_split(bp_tma_kernel<TV, false, false, true>);
     }
-    if (matched) return axial ? go(bp_tma_kernel<TP, TV, true, true, false>) : go(bp_tma_kernel<TP, TV, true, false, false>);
-    return axial ? go(bp_tma_kernel<TP, TV, false, true, false>) : go(bp_tma_kernel<TP, TV, false, false, false>);
+    if (matched) return axial ? go(bp_tma_kernel<TV, true, true, false>) : go(bp_tma_kernel<TV, true, false, false>);
+    return axial ? go(bp_tma_kernel<TV, false, true, false>) : go(bp_tma_kernel<TV, false, false, false>);
 }
 
 }  // namespace
@@ -610,17 +602,20 @@ bool bp_tma_supported(const TigrePlan* P, int pdt) {
 
 int launch_backproject_tma(TigrePlan* P, const void* proj, int pitch, int pdt, void* vol, int vdt, int matched,
                            int a0, int a1, int accumulate, cudaStream_t st) {
+    // FP32 patches only: 16-bit projections are widened first
+    if (pdt != TIGRE_F32 || (vdt != TIGRE_F32 && vdt != TIGRE_BF16))
+        return fail(TIGRE_ERR_BAD_ASSERT, "unsupported dtype pair for the staged backprojector");
     auto enc = encode_fn();
     if (!enc) return fail(TIGRE_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
     const int na = a1 - a0;
-    const size_t es = dtype_size(pdt);
+    const size_t es = sizeof(float);
     CUtensorMap tm;
     cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)P->d.nV, (cuuint64_t)na};
     cuuint64_t strides[2] = {(cuuint64_t)pitch * es, (cuuint64_t)pitch * P->d.nV * es};
-    const int BU = pdt == TIGRE_F32 ? P->bp_box_u : P->bp_box_u16;
+    const int BU = P->bp_box_u;
     cuuint32_t box[3] = {(cuuint32_t)BU, (cuuint32_t)P->bp_box_v, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(&tm, pdt == TIGRE_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+    CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                      const_cast<void*>(proj), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(TIGRE_ERR_CUDA, "cuTensorMapEncodeTiled failed");
@@ -641,9 +636,8 @@ int launch_backproject_tma(TigrePlan* P, const void* proj, int pitch, int pdt, v
     const long long skip = option(TIGRE_OPT_BP_SKIP_COPY);
     a.skip_view = (skip >= 0 && skip < na) ? (int)skip : -1;
     const bool ax = P->axial;
-    if (pdt == TIGRE_F32 && vdt == TIGRE_F32) return launch_typed<float, float>(tm, a, matched, ax, st);
-    if (pdt == TIGRE_F32 && vdt == TIGRE_BF16) return launch_typed<float, __nv_bfloat16>(tm, a, matched, ax, st);
-    return fail(TIGRE_ERR_BAD_ASSERT, "unsupported dtype pair for the staged backprojector");
+    if (vdt == TIGRE_F32) return launch_typed<float>(tm, a, matched, ax, st);
+    return launch_typed<__nv_bfloat16>(tm, a, matched, ax, st);
 }
 
 }  // namespace tigre

@@ -140,7 +140,6 @@ struct TigrePlan {
     std::vector<tigre::FrameBPK> h_bpk;
     tigre::FrameBPK* d_bpk = nullptr;
     int bp_box_u = 0, bp_box_v = 0;   // TMA patch box of the staged backprojector (0: not usable)
-    int bp_box_u16 = 0;               // box width for 16-bit projections
     int* d_status = nullptr;          // kernel error word (bounded waits that expired)
     // hardware-texture interpolated projector (TIGRE_OPT_INTERP_TEXTURE): FP32 3-D array + texture
     cudaArray_t tex_array = nullptr;
