@@ -230,83 +230,92 @@ __global__ void __launch_bounds__(256) conv_in_kernel(const float* __restrict__ 
 }
 
 // Last convolution: CIN input channels -> 1, rounded to BF16, plus the residual volume (FP32).  The
-// products run on the warp-level tensor cores with the 27 taps as output columns,
-//     P[v][t] = sum_c x[v][c] w[t][c],   out[v] = b + sum_t P[v + off(t)][t],
-// so that every input voxel is read and multiplied once instead of 27 times.  A block marches a
-// 62 x 8 tile of (x, y) down kOutZ slices: per input slice, P of its 64 x 10 halo tile goes to
-// shared memory as [tap][row][x] (pitch 66: the fragments' stores and the sums' loads are free of
-// bank conflicts), and each thread adds the nine taps of each dz into the three output slices that
-// the input slice touches.  K index 2 q + e of the low half is channel 4 q + e of a 16-channel
-// step, of the high half channel 4 q + 2 + e: a thread's operands are one 8-byte load per voxel.
-// 256^3, 16 channels: 498 us (1358 with 27 x 16 scalar FMAs and as many conversions per voxel); bound
-// by the shared-memory passes over P, 27 words written and read per voxel.
-constexpr int kOutX = 62, kOutY = 8, kOutZ = 32, kOutPitch = 66;
-constexpr size_t kOutSmem = sizeof(float) * 27 * (kOutY + 2) * kOutPitch;
+// products run on the warp-level tensor cores with the three rows dy in K and the nine taps (dz, dx) as
+// output columns,
+//     P[v][dz, dx] = sum_dy sum_c x[v + dy][c] w[dz, dy, dx][c],   out[v] = b + sum P[v + (dz, dx)][dz, dx],
+// so that every input voxel's operands are loaded once (1.5 times, with the warps' edge rows), used
+// for three rows, and nine words per voxel pass through shared memory instead of 27.  A block marches a
+// 62 x 8 tile of (x, y) down kOutZ slices: per input slice, a warp takes 16 x and four of the rows, P goes to
+// shared memory as [tap][row][x] (kOutPlane words a tap, which with the pitch leaves the fragments' stores and
+// the sums' loads free of bank conflicts), and each thread adds the three dx of each dz into the three
+// output slices that the input slice touches.  K index 2 q + e of the low half is channel 4 q + e of a
+// 16-channel step, of the high half channel 4 q + 2 + e: a thread's operands are one 8-byte load per voxel.
+// 256^3, 16 channels: 336 us (27 tap columns, one row at a time: 498); bound by the latency of the loads, all
+// issued before the first product, and of the two barriers a slice.  2 / 4 / 5 blocks per SM 433 / 489 / 552;
+// rows loaded one ahead in a window of four at 3 or 4 blocks per SM 455 / 442.
+constexpr int kOutX = 62, kOutY = 8, kOutZ = 32, kOutPitch = 66, kOutPlane = kOutY * kOutPitch + 4;
 
 template <int CIN>
-__global__ void __launch_bounds__(256) conv_out_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256, CIN <= 16 ? 3 : 1) conv_out_kernel(const __nv_bfloat16* __restrict__ x,
                                                        const __nv_bfloat16* __restrict__ w, float b,
                                                        const float* __restrict__ vol, float* __restrict__ out, int D,
                                                        int H, int W, int tx, int ty) {
     constexpr int KS = (CIN + 15) / 16;        // K steps (8 channels: one step, its high half zero)
     constexpr int CQ = CIN >= 16 ? 4 : 2;      // channels of a step that a thread holds
-    extern __shared__ float P[];               // [27][kOutY + 2][kOutPitch]
+    constexpr int RW = kOutY / 2;              // rows of a warp
+    __shared__ float P[9 * kOutPlane];         // [tap][kOutY][kOutPitch]
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q = lane & 3;
     const int bx = (int)(blockIdx.x % (unsigned)tx), bt = (int)(blockIdx.x / (unsigned)tx);
     const int x0 = bx * kOutX, y0 = bt % ty * kOutY, z0 = bt / ty * kOutZ, zend = min(z0 + kOutZ, D);
-    uint32_t wb[KS][4][2];                     // [step][tap tile][K half]
+    uint32_t wb[KS][3][2][2];                  // [step][dy][column tile][K half]
 #pragma unroll
     for (int k = 0; k < KS; ++k)
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int tap = 8 * t + g;
-            const __nv_bfloat16* src = w + (tap < 27 ? tap : 0) * CIN + 16 * k + CQ * q;
-            wb[k][t][0] = tap < 27 ? pack_bf16(src[0], src[1]) : 0u;
-            wb[k][t][1] = tap < 27 && CQ == 4 ? pack_bf16(src[CQ - 2], src[CQ - 1]) : 0u;
-        }
+        for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int n = 8 * t + g, tap = n < 9 ? (n / 3 * 3 + dy) * 3 + n % 3 : 0;
+                const __nv_bfloat16* src = w + tap * CIN + 16 * k + CQ * q;
+                wb[k][dy][t][0] = n < 9 ? pack_bf16(src[0], src[1]) : 0u;
+                wb[k][dy][t][1] = n < 9 && CQ == 4 ? pack_bf16(src[CQ - 2], src[CQ - 1]) : 0u;
+            }
     // the thread's two output voxels and their sums for slices s - 1, s, s + 1 (s: input slice)
     const int ox = tid & 63, oy = tid >> 6;    // rows oy and oy + 4
     float o0[2] = {0.f, 0.f}, o1[2] = {0.f, 0.f}, o2[2];
+    const int xb = (wid & 3) * 16, rb = (wid >> 2) * RW;
     for (int s = max(z0 - 1, 0); s <= min(zend, D - 1); ++s) {
-        // P of the (kOutY + 2) x 64 halo tile: 40 tiles of 16 voxels over 8 warps
+        uint32_t a[RW + 2][KS][2][2];          // [input row rb - 1 + j][step][voxel g / g + 8][K half]
 #pragma unroll
-        for (int i = 0; i < (kOutY + 2) * 4 / 8; ++i) {
-            const int mt = wid + 8 * i, r = mt >> 2, xb = (mt & 3) * 16;
-            const int gy = y0 + r - 1;
-            uint32_t a[KS][2][2];              // [step][row g / g + 8][K half]
+        for (int j = 0; j < RW + 2; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int gx = x0 + xb + g + 8 * h - 1;
+                const int gy = y0 + rb + j - 1, gx = x0 + xb + g + 8 * h - 1;
                 const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
                 const __nv_bfloat16* src = x + (((long)s * H + (ok ? gy : 0)) * W + (ok ? gx : 0)) * CIN + CQ * q;
 #pragma unroll
                 for (int k = 0; k < KS; ++k) {
                     if constexpr (CQ == 4) {
                         const uint2 v = ok ? __ldg(reinterpret_cast<const uint2*>(src + 16 * k)) : make_uint2(0u, 0u);
-                        a[k][h][0] = v.x;
-                        a[k][h][1] = v.y;
+                        a[j][k][h][0] = v.x;
+                        a[j][k][h][1] = v.y;
                     } else {
-                        a[k][h][0] = ok ? __ldg(reinterpret_cast<const uint32_t*>(src)) : 0u;
-                        a[k][h][1] = 0u;
+                        a[j][k][h][0] = ok ? __ldg(reinterpret_cast<const uint32_t*>(src)) : 0u;
+                        a[j][k][h][1] = 0u;
                     }
                 }
             }
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
+        for (int r = 0; r < RW; ++r)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
                 float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int k = 0; k < KS; ++k) mma_bf16(c, a[k][0][0], a[k][1][0], a[k][0][1], a[k][1][1], wb[k][t][0], wb[k][t][1]);
-                float* d = P + ((8 * t + 2 * q) * (kOutY + 2) + r) * kOutPitch + xb + g;
-                if (8 * t + 2 * q < 27) {
+                for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                    for (int k = 0; k < KS; ++k) {
+                        const uint32_t(&f)[2][2] = a[r + dy][k];
+                        mma_bf16(c, f[0][0], f[1][0], f[0][1], f[1][1], wb[k][dy][t][0], wb[k][dy][t][1]);
+                    }
+                float* d = P + (8 * t + 2 * q) * kOutPlane + (rb + r) * kOutPitch + xb + g;
+                if (t == 0 || q == 0) {        // column 8 is the last
                     d[0] = c[0];
                     d[8] = c[2];
                 }
-                if (8 * t + 2 * q + 1 < 27) {
-                    d[(kOutY + 2) * kOutPitch] = c[1];
-                    d[(kOutY + 2) * kOutPitch + 8] = c[3];
+                if (t == 0) {
+                    d[kOutPlane] = c[1];
+                    d[kOutPlane + 8] = c[3];
                 }
             }
-        }
         __syncthreads();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -314,8 +323,7 @@ __global__ void __launch_bounds__(256) conv_out_kernel(const __nv_bfloat16* __re
             if (ox < kOutX) {
                 float sum[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-                for (int t = 0; t < 27; ++t)
-                    sum[t / 9] += P[(t * (kOutY + 2) + oy + 4 * h + t / 3 % 3) * kOutPitch + ox + t % 3];
+                for (int t = 0; t < 9; ++t) sum[t / 3] += P[t * kOutPlane + (oy + 4 * h) * kOutPitch + ox + t % 3];
                 o0[h] += sum[2];   // dz = 2: input slice s is z + 1 of output slice s - 1
                 o1[h] += sum[1];
                 o2[h] = sum[0];
@@ -410,8 +418,7 @@ int tigre_unet_conv_out(const void* d_x, long Cin, const void* d_w, float b, con
     if (blocks > INT_MAX || D > INT_MAX - 64 || H > INT_MAX - 64 || W > INT_MAX - 128)
         return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_out: volume too large");
     auto go = [&](auto kern) -> int {
-        TIGRE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOutSmem));
-        kern<<<(unsigned)blocks, 256, kOutSmem, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W, (int)tx, (int)ty);
+        kern<<<(unsigned)blocks, 256, 0, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W, (int)tx, (int)ty);
         TIGRE_LAUNCHED();
         return TIGRE_SUCCESS;
     };
