@@ -3,15 +3,17 @@
 //
 // Activations are channels-last volumes x[D][H][W][C] (BF16); weights w[Cout][27*Cin] with
 // the tap index t = (dz*3 + dy)*3 + dx major and the input channel minor; zero padding of 1,
-// stride 1.  Each convolution is an implicit GEMM done in two steps:
-//   im2col:   col[v][t*Cin + c] = x at voxel v shifted by tap t      (M = D*H*W rows, K = 27*Cin)
-//   forward:  y[v][co]  = relu?(sum_k col[v][k] w[co][k] + b[co])   (M x N = Cout, K)
-//   data:     dcol[v][k] = sum_co dy[v][co] w[co][k];  dx = col2im(dcol) (gather over taps)
-//   weight:   dw[co][k] += sum_v dy[v][co] col[v][k]                 (split over v, FP32 atomics)
+// stride 1.  Layers whose channel counts are multiples of 16 run elsewhere: forward and data gradient on
+// the halo-tile kernel (conv3d_tc.cu), weight gradient on staged voxel tiles (conv3d_wgrad.cu).  This
+// file holds the entry points and the paths for all other counts:
+//   forward: per-step gathers into tcgen05, or the warp-level implicit GEMM, for Cin a multiple of 8;
+//   im2col:  col[v][t*Cin + c] = x at voxel v shifted by tap t      (M = D*H*W rows, K = 27*Cin), then
+//   forward: y[v][co]  = relu?(sum_k col[v][k] w[co][k] + b[co])   (M x N = Cout, K)
+//   data:    dcol[v][k] = sum_co dy[v][co] w[co][k];  dx = col2im(dcol) (gather over taps)
+//   weight:  dw[co][k] += sum_v dy[v][co] col[v][k]                 (split over v, added in a fixed order)
 // The GEMM stages 64 x 64 output tiles through shared memory in K steps of 32 and runs them on
 // 16 x 16 x 16 BF16 warp MMA tiles (8 warps, each a 16 x 32 strip), zero-filling ragged edges,
-// so any M, N, K work.  This is the warp-level (mma.sync) tensor-core path; moving the GEMM to
-// tcgen05 with TMEM accumulators is the next step for this part.
+// so any M, N, K work.
 
 #include <cuda_bf16.h>
 #include <mma.h>
