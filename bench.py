@@ -597,7 +597,7 @@ TRAFFIC_SOURCE = ("dram__bytes_read.sum + dram__bytes_write.sum of a single-pass
 # instructions and shared-memory wavefronts per view of the launch.  The Siddon kernel's DRAM
 # traffic is 0.6 % of its algorithmic bytes: it is bound by instruction issue and on-chip load
 # latency; the backprojector reads its taps from shared memory: bound by shared wavefronts and issue.
-PROFILED = {"siddon": {"warp_inst_per_view": 6.127e9 / 36, "source": "profiles/siddon_cells_512cube_36views.txt"},
+PROFILED = {"siddon": {"warp_inst_per_view": 5.401e9 / 36, "source": "profiles/siddon_cells_512cube_36views.txt"},
             "bp": {"warp_inst_per_view": 2.949e9 / 36, "wavefronts_per_view": 7.605e8 / 36,
                    "ideal_wavefronts_per_view": 512 ** 3 * 4 / 32,
                    "source": "profiles/bp_tma_matched_512cube_36views.txt"}}
@@ -651,22 +651,23 @@ def time_ops(P, plan, vol, proj, reps=3):
                             math.prod(NVOX) * TV_ITERS, "Gvox-iter/s")
     cases["tv_piccs_f32"] = (lambda: P.tv_piccs_(tv_vol, tv_prior, TV_ALPHA, 0.5, TV_ITERS, tv_work),
                              math.prod(NVOX) * TV_ITERS, "Gvox-iter/s")
+    from tigre_b200 import _native as native
     from tigre_b200.utilities.im_3d_denoise import tv_denoise_device
-    prox_work = torch.empty(5 * NVOX[1] * NVOX[2] * (NVOX[0] + 2), dtype=torch.float32, device=vol.device)
+    prox_work = torch.empty(int(native.lib().tigre_tv_denoise_fused_floats(NVOX[2], NVOX[1], NVOX[0])), dtype=torch.float32,
+                            device=vol.device)
     cases["tv_denoise_f32"] = (lambda: tv_denoise_device(vol, TV_ITERS, 15.0, prox_work), math.prod(NVOX) * TV_ITERS,
                                "Gvox-iter/s")
     # algorithmic bytes per launch (FP32 / BF16 element bytes e): interpolated: 8 corner reads per
     # sample inside the volume + one output write per ray; backprojection: 4 bilinear taps per
     # voxel update + one volume write; POCS-TV: 12 B per voxel and step (norm pass reads f,
     # update pass reads f and writes f'; AwTV the same; PICCS 20 B, the prior read in both passes);
-    # TV proximal: 52 B per voxel and iteration (u pass reads f, u, p and writes u; p pass reads
-    # u, p and writes p)
+    # TV proximal: 36 B per voxel and iteration (one pass reads f, u, p and writes u, p)
     nsamp = P.interp_samples(plan)
     nvox = math.prod(NVOX)
     alg = {"ax_interpolated_f32": nsamp * 8 * 4 + rays * 4, "ax_interpolated_bf16": nsamp * 8 * 2 + rays * 2,
            "atb_fdk_f32": upd * 4 * 4 + nvox * 4, "atb_matched_bf16": upd * 4 * 2 + nvox * 2,
            "atb_fdk_bf16": upd * 4 * 2 + nvox * 2, "tv_pocs_f32": nvox * 12 * TV_ITERS,
-           "tv_denoise_f32": nvox * 52 * TV_ITERS, "tv_awtv_f32": nvox * 12 * TV_ITERS,
+           "tv_denoise_f32": nvox * 36 * TV_ITERS, "tv_awtv_f32": nvox * 12 * TV_ITERS,
            "tv_piccs_f32": nvox * 20 * TV_ITERS}
     out = {}
     for name, (fn, units, unit) in cases.items():
