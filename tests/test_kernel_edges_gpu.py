@@ -104,6 +104,28 @@ def test_siddon_cell_lists(xy, nv, mode):
     _close(got.cpu().numpy(), O.ax(vol, geo, ang.astype(np.float32), "Siddon"))
 
 
+@pytest.mark.parametrize("nz,vox", [(20, 0.1), (20, 0.3), (24, 1.1)])
+@pytest.mark.parametrize("nv", [5, 65, 257])
+def test_siddon_row_beside_a_slice_plane(nz, vox, nv):
+    """An odd number of rows over an even number of slices: the central row runs in the middle plane, and
+    with a voxel size that FP32 does not hold that plane comes out less than half an FP32 step of z above
+    the row.  Such a row counts as on the plane and reads the slice above, in its whole length."""
+    import torch
+    from tigre_b200 import projectors as P
+    side = np.float64(np.float32(nz * vox)) / 2 / np.float64(np.float32(vox))
+    assert 0 < nz / 2 - side < 0.5 * float(np.spacing(np.float32(nz / 2 + 3.99)))   # four slices of pad and more
+    shape = (nz, 18, 22)
+    geo = cone_geometry(shape, [n * vox for n in shape], (nv, 9), (vox * 40.0 / nv, vox * 4.0), DSO=1000.0 * vox,
+                        DSD=1536.0 * vox)
+    ang = G.angles(7)
+    vol = np.random.default_rng(nz).random(shape, dtype=np.float32)
+    got = P.ax(torch.from_numpy(vol).cuda(), _plan(geo, ang), "Siddon").cpu().numpy()
+    ref = O.ax(vol, geo, ang, "Siddon")
+    vol[nz // 2 - 1] = vol[nz // 2]      # the row's value, whichever of the two slices the oracle takes
+    ref[:, nv // 2] = O.ax(vol, geo, ang, "Siddon")[:, nv // 2]
+    _close(got, ref)
+
+
 @pytest.mark.parametrize("nv", [24, 100, 256])
 def test_siddon_copy_beyond_one_window(nv):
     """A working copy larger than 4 GB, so that its addresses differ in their high words, against the

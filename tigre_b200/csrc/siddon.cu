@@ -372,19 +372,20 @@ __global__ void __launch_bounds__(128, 6) siddon_columns_kernel(SiddonArgs p) {
 // siddon_columns_kernel, but the z state is not stepped: with z(alpha) = zA + alpha*rz
 // the slice at the end b of each xy cell is floor(z(b)), and since at most one z plane
 // lies inside the cell, its contribution is
-//     seg * v(z_start) + (z(b) - z_plane) / rz * (v(z_end) - v(z_start)).
-// z is measured from the first plane that the ray meets, so that z(b) - z_plane is a
-// difference of small numbers: its error is that of alpha, times rz.  The two sums over the
-// cells are kept apart and the division is done once per ray.  Without a crossing
-// v(z_end) = v(z_start) and the second term is zero, so every cell of every row runs the same
-// branch-free code, two rows at a time in packed FP32x2.  The floor is a round-toward-zero add of
-// 1.5*2^23 + the plane's index (z is kept positive by the pads), and its float bits index the
-// column directly.  The pads (at least the largest z extent of any ray inside the xy box, from
-// the host) make every index valid without clamping: a ray whose z range misses the volume reads
-// one zero slice.
+//     seg * v(z_start) + (b - alpha_k) * (v(z_end) - v(z_start)),
+// where alpha_k is the crossing, taken in alpha space from the crossing count
+// (alpha_k = tz0 + (z_end - q) / rz, exact small integers in the difference).  Without a
+// crossing v(z_end) = v(z_start) and the second term is zero, so every cell of every row
+// runs the same branch-free code on the FMA pipe, two rows at a time in packed FP32x2.
+// The floor is a round-toward-zero add of 1.5*2^23 (z is kept positive by the pads), and
+// its float bits index the column directly.  The pads (at least the largest z extent of
+// any ray inside the xy box, from the host) make every index valid without clamping:
+// a ray whose z range misses the volume reads one zero slice.  z is held with its pad in FP32:
+// a ray nearer to a slice plane than half an FP32 step there counts as on it, and reads the slice
+// above, all along if it runs beside the plane.
 //
 // What bounds it is instructions: the packed FP32 operations take two cycles each on one pipe,
-// 7 per row pair and cell, beside one load per row and end of the cell and the integer work that
+// 8 per row pair and cell, beside one load per row and end of the cell and the integer work that
 // addresses it.  So everything else is kept out of the loop over cells:
 //  * the cells are the same for all rows of a warp, so its lanes merge the x and y crossings 32
 //    cells at a time, one crossing each, into a list in shared memory, and the loop reads the end,
@@ -430,6 +431,7 @@ struct CellList {
     int next_x, next_y;           // crossings used by this list and the earlier ones
     float t0x, dtx, inv_dx, t0y, dty, inv_dy, T;   // the crossings and the exit
     int nx, ny, cell0, dcx, dcy;                   // their numbers; first cell, steps
+    double lxy;                                    // squared length in xy, for the end
 };
 
 template <typename TP, int R, bool WINDOW>
@@ -488,7 +490,7 @@ __global__ void __launch_bounds__(32 * kCellWarps, (R >= 8 ? 16 : 20) / kCellWar
     const float T = (float)Td;
     const double P = (double)p.zpad;
     // ---- per-row z state, rows (2h, 2h+1) packed in .x/.y ----
-    float2 zA[H], rz[H], Q[H], nK[H], sv[H], sd[H];
+    float2 zA[H], rz[H], nm[H], nQ[H], ntz0[H], sum[H];
     uint64_t ad[R];                                    // WINDOW: address of the row's voxel; else its offset in the column
     const uint32_t colb = (uint32_t)(p.nZ + 2 * p.zpad) * 4u;
 #pragma unroll
@@ -506,29 +508,35 @@ __global__ void __launch_bounds__(32 * kCellWarps, (R >= 8 ? 16 : 20) / kCellWar
             live = false;
             if (p.status) atomicOr(p.status, 2);
         }
-        // first plane q; index q + floor(z); the plane just crossed is floor(z), or floor(z) + 1 downwards
-        float zaf = 0.5f, rzf = 0.f, qf = (float)(P - 1.0), up = 0.f;
+        float zaf = (float)(P - 0.5), rzf = 0.f, m = 0.f, q = 0.f, tz = 0.f;
         if (live) {
-            const double q = floor(za) + (rzd > 0.0 ? 1.0 : 0.0);
-            zaf = (float)(za - q);
+            zaf = (float)za;
             rzf = (float)rzd;
-            qf = (float)q;
-            up = rzd > 0.0 ? 0.f : 1.f;
+            const float zs = __fadd_rz(zaf, kMagic) - kMagic;   // floor(zA) as the loop computes it
+            if (rzd > 0.0) {
+                q = zs + 1.f;
+                tz = (float)(((double)zs + 1.0 - za) / rzd);
+                m = (float)(1.0 / rzd);
+            } else if (rzd < 0.0) {
+                q = zs - 1.f;
+                tz = (float)(((double)zs - za) / rzd);
+                m = (float)(1.0 / rzd);
+            }
         }
-        const float Qr = kMagic + qf;
-        ad[r] = (uint64_t)(__float_as_uint(__fadd_rz(zaf, Qr)) - kMagicBits) * 4u + (WINDOW ? (uintptr_t)p.vol_x : 0u);
+        ad[r] = (uint64_t)(__float_as_uint(__fadd_rz(zaf, kMagic)) - kMagicBits) * 4u + (WINDOW ? (uintptr_t)p.vol_x : 0u);
         if (r & 1) {
-            zA[r >> 1].y = zaf; rz[r >> 1].y = rzf; Q[r >> 1].y = Qr; nK[r >> 1].y = up - Qr;
-            sv[r >> 1].y = 0.f; sd[r >> 1].y = 0.f;
+            zA[r >> 1].y = zaf; rz[r >> 1].y = rzf; nm[r >> 1].y = -m; nQ[r >> 1].y = -(kMagic + q);
+            ntz0[r >> 1].y = -tz; sum[r >> 1].y = 0.f;
         } else {
-            zA[r >> 1].x = zaf; rz[r >> 1].x = rzf; Q[r >> 1].x = Qr; nK[r >> 1].x = up - Qr;
-            sv[r >> 1].x = 0.f; sd[r >> 1].x = 0.f;
+            zA[r >> 1].x = zaf; rz[r >> 1].x = rzf; nm[r >> 1].x = -m; nQ[r >> 1].x = -(kMagic + q);
+            ntz0[r >> 1].x = -tz; sum[r >> 1].x = 0.f;
         }
     }
     if (lane == 0) {
         list.t0x = ax.t0; list.dtx = ax.dt; list.inv_dx = nx ? 1.f / ax.dt : 0.f; list.nx = nx; list.dcx = ax.step * p.nY;
         list.t0y = ay.t0; list.dty = ay.dt; list.inv_dy = ny ? 1.f / ay.dt : 0.f; list.ny = ny; list.dcy = ay.step;
         list.T = T; list.cell0 = ax.i * p.nY + ay.i;
+        list.lxy = rx * rx * p.dVX * p.dVX + ry * ry * p.dVY * p.dVY;
     }
     if (lane == 0) {
         list.b[kListCells] = 0.f;
@@ -604,17 +612,18 @@ __global__ void __launch_bounds__(32 * kCellWarps, (R >= 8 ? 16 : 20) / kCellWar
         asm("{\n.reg .b32 lo, hi;\nmov.b64 {lo, hi}, %0;\nmov.b64 %0, {%1, hi};\n}" : "+l"(x) : "r"(lo));
         return ld(x);
     };
-    float2 g[H], v0[H], v1[H], seg2;
+    float2 d[H], v0[H], v1[H], seg2;
     auto front = [&](int h, float2 b2, uint2 col) {
         const float2 z = __ffma2_rn(b2, rz[h], zA[h]);
-        const float2 t = __fadd2_rz(z, Q[h]);
-        g[h] = __ffma2_rn(__fadd2_rn(t, nK[h]), pk(-1.f), z);     // z - plane; the plane is exact
+        const float2 t = __fadd2_rz(z, pk(kMagic));                // kMagic + floor(z(b))
+        const float2 kq = __fadd2_rn(t, nQ[h]);                    // z_end - q, exact
+        d[h] = __fadd2_rn(b2, __ffma2_rn(kq, nm[h], ntz0[h]));     // b - alpha_k
         v0[h] = pk(load0(ad[2 * h], col), load0(ad[2 * h + 1], col));
         v1[h] = pk(load1(ad[2 * h], t.x, col), load1(ad[2 * h + 1], t.y, col));
     };
     auto back = [&](int h) {
-        sv[h] = __ffma2_rn(seg2, v0[h], sv[h]);
-        sd[h] = __ffma2_rn(g[h], __ffma2_rn(v0[h], pk(-1.f), v1[h]), sd[h]);
+        sum[h] = __ffma2_rn(seg2, v0[h], sum[h]);
+        sum[h] = __ffma2_rn(d[h], __ffma2_rn(v0[h], pk(-1.f), v1[h]), sum[h]);
     };
     build(0);
     {
@@ -641,7 +650,7 @@ __global__ void __launch_bounds__(32 * kCellWarps, (R >= 8 ? 16 : 20) / kCellWar
     }
 #pragma unroll
     for (int h = 0; h < H; ++h) back(h);
-    const double lxy = rx * rx * p.dVX * p.dVX + ry * ry * p.dVY * p.dVY;
+    const double lxy = list.lxy;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int v = vbase + 32 * r;
@@ -651,10 +660,8 @@ __global__ void __launch_bounds__(32 * kCellWarps, (R >= 8 ? 16 : 20) / kCellWar
             double rzd = fma(pv, F.dv[2], fma((double)u, F.du[2], F.o[2])) - szr;
             if (fabs(rzd) < 0.001) rzd = 0.0;
             const float len = (float)sqrt(lxy + rzd * rzd * p.dVZ * p.dVZ);
-            const float rzr = (r & 1) ? rz[r >> 1].y : rz[r >> 1].x;    // 0 also for a ray that misses the volume
-            const float m = rzr != 0.f ? (float)(1.0 / rzd) : 0.f;
-            const float s = fmaf(m, (r & 1) ? sd[r >> 1].y : sd[r >> 1].x, (r & 1) ? sv[r >> 1].y : sv[r >> 1].x);
-            out[(size_t)v * p.nU] = from_f32<TP>(s * len);
+            const float sr = (r & 1) ? sum[r >> 1].y : sum[r >> 1].x;
+            out[(size_t)v * p.nU] = from_f32<TP>(sr * len);
         }
     }
 }
