@@ -297,3 +297,40 @@ def test_first_and_last_convolution(c, D, H, W):
     N.check(L.tigre_unet_conv_out(p(x), c, p(wo), 0.25, p(vol), p(out), D, H, W, None), "conv_out")
     ref = _conv64(x, wo, 1)[0, 0] + 0.25
     assert float((out.double() - vol.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()) + 1e-6
+
+
+@pytest.mark.parametrize("c", [8, 16, 32])
+@pytest.mark.parametrize("D,H,W", [(1, 1, 1), (8, 8, 8), (17, 9, 65), (33, 40, 31), (70, 17, 33)])
+def test_first_and_last_convolution_order(c, D, H, W):
+    """Every sum starts at the bias and takes taps, then channels, in order by FP32 fused multiply-adds: the
+    same bits.  (BF16 products are exact in FP64 and so is their sum with an FP32 value 2^29 times larger
+    or smaller at most, so that one rounding to FP32 is the fused operation.)"""
+    import torch
+    from tigre_b200 import _native as N
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    L, p = N.lib(), lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    shifts = [(t // 9, t // 3 % 3, t % 3) for t in range(27)]
+
+    def taps(v):     # (27, D, H, W, ...) of the zero-padded volume, in FP64
+        q = torch.zeros((D + 2, H + 2, W + 2) + v.shape[3:], dtype=torch.float64, device="cuda")
+        q[1:-1, 1:-1, 1:-1] = v.double()
+        return [q[z:z + D, y:y + H, x:x + W] for z, y, x in shifts]
+    vol = torch.randn((D, H, W), device="cuda", generator=g)
+    w = torch.randn((c, 27), device="cuda", generator=g).bfloat16()
+    b = torch.randn(c, device="cuda", generator=g)
+    y = torch.empty((D, H, W, c), dtype=torch.bfloat16, device="cuda")
+    N.check(L.tigre_unet_conv_in(p(vol), p(w), p(b), p(y), D, H, W, c, 1, None), "conv_in")
+    acc = b.expand(D, H, W, c)
+    for t, v in enumerate(taps(vol.bfloat16())):
+        acc = (acc.double() + v[..., None] * w[:, t].double()).float()
+    assert torch.equal(y, acc.relu().bfloat16())
+    x = torch.randn((D, H, W, c), device="cuda", generator=g).bfloat16()
+    wo = torch.randn((27, c), device="cuda", generator=g).bfloat16()
+    out = torch.empty_like(vol)
+    N.check(L.tigre_unet_conv_out(p(x), c, p(wo), 0.25, p(vol), p(out), D, H, W, None), "conv_out")
+    acc = torch.full_like(vol, 0.25)
+    for t, v in enumerate(taps(x)):
+        for k in range(c):
+            acc = (acc.double() + v[..., k] * wo[t, k].double()).float()
+    assert torch.equal(out, vol + acc.bfloat16().float())

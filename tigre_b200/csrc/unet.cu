@@ -1,8 +1,10 @@
 // The glue of the warm-start U-Net's inference pass, fused so that each step is one pass over
 // HBM (channels-last BF16 activations, FP32 arithmetic):
 //   tigre_unet_pool2      2x2x2 average pooling                  (read 8 voxels, write 1)
-//   tigre_unet_up_concat  nearest 2x upsampling of the deeper level concatenated with the skip
-//                         connection along channels              (one write of the decoder input)
+//   tigre_unet_up2        nearest 2x upsampling of the deeper level, which the decoder's convolution
+//                         reads beside the skip connection       (read 1 voxel, write 8)
+//   tigre_unet_up_concat  the same concatenated with the skip connection along channels, where the
+//                         convolution does not take two inputs   (one write of the decoder input)
 //   tigre_unet_conv_in    the first 3x3x3 convolution (one input channel, FP32 volume rounded to
 //                         BF16 on the fly, FP32 accumulation, bias, ReLU)
 //   tigre_unet_conv_out   the last 3x3x3 convolution (one output channel) rounded to BF16 as the
@@ -101,127 +103,105 @@ __global__ void __launch_bounds__(256) up2_kernel(const uint4* __restrict__ low,
     }
 }
 
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
-}
-
-// First convolution: one input channel (vol, FP32, rounded to BF16), COUT outputs, as warp-level
-// m16n8k16 products of 16 voxels along x with the taps as K.  Per (dz, dy) row the three dx taps
-// take two K pairs, (x-1, x) and (x+1, -), so that an operand register is one 32-bit word of the
-// staged row; the row is kept twice, the second copy shifted by one voxel, which makes the pair of
-// any x an aligned word.  18 of 24 K pairs carry weights; the others and the unused halves are
-// zeroed on both sides.  A block marches a 64 x 8 tile of (x, y) down kInZ slices, three staged at a
-// time; output column c of tile t is channel 2 NT (c / 2) + 2 t + c % 2, so a thread stores
-// 4 NT contiguous bytes.
-// 256^3, 16 channels: 205 us, 604 MB written and read at 2.9 TB/s (scalar FMAs, 27 bounds-tested loads a
-// voxel: 806 us); bound by the shared-memory loads of the operands and the staging.
-constexpr int kInX = 64, kInY = 8, kInZ = 16;
-constexpr int kInWords = kInX / 2 + 2;                 // words of one staged row and copy
-constexpr int kInPitch = 2 * kInWords + 1;             // both copies (odd: rows fall in other banks)
+// First convolution: one input channel (vol, FP32, rounded to BF16), COUT outputs.  The sum of an
+// output starts from its bias and takes the 27 taps in order, each by one FP32 fused multiply-add:
+// what the network computes behind it depends on every rounding here (the BF16 steps of 14 layers), so
+// the order is part of the result, and the tensor cores, which sum in one of their own, are not used.
+// A block marches a 32 x 16 tile of (x, y) down a chunk of slices, three staged at a time and the next one
+// on its way in registers; a thread owns four rows of one x and 16 channels, so that a tap's weights (one
+// broadcast 16-byte load per four) serve four voxels and a voxel up to nine taps, two channels to an
+// instruction.  Bound by the FP32 pipe, 27 COUT multiply-adds a voxel: 256^3, 16 channels 322 us, 201 at its
+// full rate (one voxel a thread with 27 bounds-tested loads 785; on the tensor cores, in their order, 203);
+// 64^3 11 us (19).  Four blocks per SM 374 (spills); two rows a thread at 5 or 6 blocks 341 / 367.
+constexpr int kInX = 32, kInY = 16, kInRows = 4, kInBlocks = 3;
+constexpr int kInThreads = kInX * kInY / kInRows;
+constexpr int kInHalo = (kInX + 2) * (kInY + 2), kInFetch = (kInHalo + kInThreads - 1) / kInThreads;
 
 template <int COUT>
-__global__ void __launch_bounds__(256) conv_in_kernel(const float* __restrict__ vol, const __nv_bfloat16* __restrict__ w,
-                                                      const float* __restrict__ b, __nv_bfloat16* __restrict__ y,
-                                                      int D, int H, int W, int tx, int ty, int relu) {
-    constexpr int NT = COUT / 8;
-    __shared__ uint32_t ring[3][kInY + 2][kInPitch];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q = lane & 3;
+__global__ void __launch_bounds__(kInThreads, kInBlocks) conv_in_kernel(const float* __restrict__ vol,
+                                                                const __nv_bfloat16* __restrict__ w,
+                                                                const float* __restrict__ b, __nv_bfloat16* __restrict__ y,
+                                                                int D, int H, int W, int tx, int ty, int zc, int relu) {
+    constexpr int CG = COUT < 16 ? COUT : 16;   // channels of a thread at a time
+    __shared__ float ring[3][kInHalo];
+    __shared__ __align__(16) float sw[27][COUT];
+    __shared__ float sb[COUT];
+    const int tid = threadIdx.x, lx = tid % kInX, ly = tid / kInX * kInRows;
     const int bx = (int)(blockIdx.x % (unsigned)tx), bt = (int)(blockIdx.x / (unsigned)tx);
-    const int x0 = bx * kInX, y0 = bt % ty * kInY, z0 = bt / ty * kInZ, zend = min(z0 + kInZ, D);
-    auto channel = [](int t, int c) { return 2 * NT * (c >> 1) + 2 * t + (c & 1); };
-    // weights: K pair slot s = 8 kstep + 4 half + q holds taps (2 (s % 2), 2 (s % 2) + 1) of row s / 2
-    uint32_t wb[3][2][NT];
-    float bias[NT][2];
+    const int x0 = bx * kInX, y0 = bt % ty * kInY, z0 = bt / ty * zc, zend = min(z0 + zc, D);
+    for (int i = tid; i < 27 * COUT; i += kInThreads) sw[i % 27][i / 27] = __bfloat162float(w[i]);
+    for (int i = tid; i < COUT; i += kInThreads) sb[i] = b ? b[i] : 0.f;
+    float next[kInFetch];
+    auto fetch = [&](int z) {
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int s = 8 * k + 4 * h + q, row = s >> 1;
-                const __nv_bfloat16* src = w + channel(t, g) * 27 + row * 3;
-                const __nv_bfloat16 zero = __float2bfloat16(0.f);
-                wb[k][h][t] = row >= 9 ? 0u : (s & 1) ? pack_bf16(src[2], zero) : pack_bf16(src[0], src[1]);
-            }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) bias[t][e] = b ? b[channel(t, 2 * q + e)] : 0.f;
-    }
-    // stages slice z: word j of copy 0 = (v[2j], v[2j+1]), of copy 1 = (v[2j+1], v[2j+2]), v[0] at x0 - 1
-    auto stage = [&](int z) {
-        const bool zin = z >= 0 && z < D;
-        uint32_t(*dst)[kInPitch] = ring[(z + 3) % 3];
-        for (int e = tid; e < (kInY + 2) * kInWords; e += 256) {
-            const int r = e / kInWords, j = e - r * kInWords, gy = y0 + r - 1;
-            __nv_bfloat16 v[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int gx = x0 - 1 + 2 * j + k;
-                const bool ok = zin && gy >= 0 && gy < H && gx >= 0 && gx < W;
-                v[k] = __float2bfloat16(ok ? __ldg(vol + ((long)z * H + gy) * W + gx) : 0.f);
-            }
-            dst[r][j] = pack_bf16(v[0], v[1]);
-            dst[r][kInWords + j] = pack_bf16(v[1], v[2]);
+        for (int k = 0; k < kInFetch; ++k) {
+            const int e = tid + k * kInThreads, gy = y0 + e / (kInX + 2) - 1, gx = x0 + e % (kInX + 2) - 1;
+            const bool ok = e < kInHalo && z >= 0 && z < D && gy >= 0 && gy < H && gx >= 0 && gx < W;
+            next[k] = ok ? __ldg(vol + ((long)z * H + gy) * W + gx) : 0.f;
         }
     };
-    stage(z0 - 1);
-    stage(z0);
+    auto put = [&](int z) {
+#pragma unroll
+        for (int k = 0; k < kInFetch; ++k) {
+            const int e = tid + k * kInThreads;
+            if (e < kInHalo) ring[(z + 3) % 3][e] = __bfloat162float(__float2bfloat16(next[k]));
+        }
+    };
+    fetch(z0 - 1);
+    put(z0 - 1);
+    fetch(z0);
+    put(z0);
+    fetch(z0 + 1);
     for (int z = z0; z < zend; ++z) {
-        stage(z + 1);
+        put(z + 1);
         __syncthreads();
-        const int gy = y0 + wid;
-        if (gy < H) {
-            const uint32_t* rows[3][2];   // this thread's K pair slots
-            uint32_t mask[3][2];
+        fetch(z + 2);
+        const int gx = x0 + lx;
+#pragma unroll 1
+        for (int cg = 0; cg < COUT; cg += CG) {
+            float2 acc[kInRows][CG / 2];
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
+            for (int r = 0; r < kInRows; ++r)
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int s = 8 * k + 4 * h + q, row = min(s >> 1, 8);
-                    rows[k][h] = &ring[(z + row / 3 + 2) % 3][wid + row % 3][(s & 1) + (g & 1) * kInWords + (g >> 1)];
-                    mask[k][h] = s >= 18 ? 0u : (s & 1) ? 0xffffu : 0xffffffffu;
-                }
-            __nv_bfloat16* o = y + (((long)z * H + gy) * W + x0) * COUT;
+                for (int c = 0; c < CG / 2; ++c) acc[r][c] = make_float2(sb[cg + 2 * c], sb[cg + 2 * c + 1]);
+#pragma unroll 1
+            for (int dz = 0; dz < 3; ++dz) {
+                const float* in = &ring[(z + dz + 2) % 3][ly * (kInX + 2) + lx];
+                float v[kInRows + 2][3];
 #pragma unroll
-            for (int m = 0; m < kInX / 16; ++m) {
-                if (x0 + 16 * m >= W) break;
-                float c[NT][4];
+                for (int r = 0; r < kInRows + 2; ++r)
 #pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    c[t][0] = c[t][2] = bias[t][0];
-                    c[t][1] = c[t][3] = bias[t][1];
-                }
+                    for (int dx = 0; dx < 3; ++dx) v[r][dx] = in[r * (kInX + 2) + dx];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const uint32_t a0 = rows[k][0][8 * m] & mask[k][0], a1 = rows[k][0][8 * m + 4] & mask[k][0];
-                    const uint32_t a2 = rows[k][1][8 * m] & mask[k][1], a3 = rows[k][1][8 * m + 4] & mask[k][1];
+                for (int t = 0; t < 9; ++t) {
+                    const float4* wt = reinterpret_cast<const float4*>(&sw[9 * dz + t][cg]);
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) mma_bf16(c[t], a0, a1, a2, a3, wb[k][0][t], wb[k][1][t]);
-                }
+                    for (int c = 0; c < CG / 4; ++c) {
+                        const float4 q = wt[c];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int x = 16 * m + g + 8 * h;
-                    if (x0 + x < W) {
-                        uint32_t v[NT];
-#pragma unroll
-                        for (int t = 0; t < NT; ++t) {
-                            const float lo = relu ? fmaxf(c[t][2 * h], 0.f) : c[t][2 * h];
-                            const float hi = relu ? fmaxf(c[t][2 * h + 1], 0.f) : c[t][2 * h + 1];
-                            const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
-                            v[t] = *reinterpret_cast<const uint32_t*>(&p);
+                        for (int r = 0; r < kInRows; ++r) {
+                            const float2 in2 = make_float2(v[r + t / 3][t % 3], v[r + t / 3][t % 3]);
+                            acc[r][2 * c] = __ffma2_rn(make_float2(q.x, q.y), in2, acc[r][2 * c]);
+                            acc[r][2 * c + 1] = __ffma2_rn(make_float2(q.z, q.w), in2, acc[r][2 * c + 1]);
                         }
-                        uint32_t* dst = reinterpret_cast<uint32_t*>(o + (long)x * COUT) + NT * q;
-                        if constexpr (NT == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
-                        else if constexpr (NT == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(v[0], v[1]);
-                        else dst[0] = v[0];
                     }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kInRows; ++r) {
+                const int gy = y0 + ly + r;
+                if (gx >= W || gy >= H) continue;
+                uint4* o = reinterpret_cast<uint4*>(y + (((long)z * H + gy) * W + gx) * COUT + cg);
+#pragma unroll
+                for (int c = 0; c < CG / 8; ++c) {
+                    float f[8];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 a = acc[r][4 * c + j];
+                        f[2 * j] = relu ? fmaxf(a.x, 0.f) : a.x;
+                        f[2 * j + 1] = relu ? fmaxf(a.y, 0.f) : a.y;
+                    }
+                    o[c] = f_to_bf8(f);
                 }
             }
         }
@@ -229,119 +209,122 @@ __global__ void __launch_bounds__(256) conv_in_kernel(const float* __restrict__ 
     }
 }
 
-// Last convolution: CIN input channels -> 1, rounded to BF16, plus the residual volume (FP32).  The
-// products run on the warp-level tensor cores with the three rows dy in K and the nine taps (dz, dx) as
-// output columns,
-//     P[v][dz, dx] = sum_dy sum_c x[v + dy][c] w[dz, dy, dx][c],   out[v] = b + sum P[v + (dz, dx)][dz, dx],
-// so that every input voxel's operands are loaded once (1.5 times, with the warps' edge rows), used
-// for three rows, and nine words per voxel pass through shared memory instead of 27.  A block marches a
-// 62 x 8 tile of (x, y) down kOutZ slices: per input slice, a warp takes 16 x and four of the rows, P goes to
-// shared memory as [tap][row][x] (kOutPlane words a tap, which with the pitch leaves the fragments' stores and
-// the sums' loads free of bank conflicts), and each thread adds the three dx of each dz into the three
-// output slices that the input slice touches.  K index 2 q + e of the low half is channel 4 q + e of a
-// 16-channel step, of the high half channel 4 q + 2 + e: a thread's operands are one 8-byte load per voxel.
-// 256^3, 16 channels: 336 us (27 tap columns, one row at a time: 498); bound by the latency of the loads, all
-// issued before the first product, and of the two barriers a slice.  2 / 4 / 5 blocks per SM 433 / 489 / 552;
-// rows loaded one ahead in a window of four at 3 or 4 blocks per SM 455 / 442.
-constexpr int kOutX = 62, kOutY = 8, kOutZ = 32, kOutPitch = 66, kOutPlane = kOutY * kOutPitch + 4;
+// Last convolution: CIN input channels -> 1, rounded to BF16, plus the residual volume (FP32).  The sum
+// starts from the bias and takes the taps in order and a tap's channels in order, by FP32 fused
+// multiply-adds (as the first convolution, for the same reason).  A block marches a 32 x 16 tile of (x, y)
+// down a chunk of slices, one input slice staged and the next on its way; a slice's 9 CIN products go
+// to three output slices at once, whose sums a thread carries for four neighbouring x: the weights of the
+// three dz are one broadcast 16-byte load for 12 multiply-adds, and a staged voxel is read three times instead of 27.
+// The staged voxels are kept in planes of eight channels, every fourth x together, which makes the
+// 16-byte loads of eight threads one 128-byte run.  Bound by instruction issue, 27 CIN multiply-adds and
+// 9 CIN conversions an output voxel: 256^3, 16 channels 494 us (one voxel a thread 1362; on the tensor cores 336),
+// 64^3 29 us (31).  3 / 5 blocks per SM 530 / 515; two voxels to an instruction, which doubles the weights'
+// loads, 510 to 569.
+constexpr int kOutX = 32, kOutY = 16, kOutV = 4, kOutThreads = kOutX * kOutY / kOutV;
+constexpr int out_blocks(int cin) { return cin <= 16 ? 4 : 2; }       // resident blocks per SM
+constexpr int kOutRow = kOutV * (kOutX / kOutV + 1);                  // 16-byte places of a staged row
+constexpr int out_plane() { return (kOutY + 2) * kOutRow; }           // ... of a plane
+constexpr size_t out_smem(int cin) { return 16 * (size_t)(2 * cin / 8 * out_plane() + 9 * cin); }
 
 template <int CIN>
-__global__ void __launch_bounds__(256, CIN <= 16 ? 3 : 1) conv_out_kernel(const __nv_bfloat16* __restrict__ x,
-                                                       const __nv_bfloat16* __restrict__ w, float b,
-                                                       const float* __restrict__ vol, float* __restrict__ out, int D,
-                                                       int H, int W, int tx, int ty) {
-    constexpr int KS = (CIN + 15) / 16;        // K steps (8 channels: one step, its high half zero)
-    constexpr int CQ = CIN >= 16 ? 4 : 2;      // channels of a step that a thread holds
-    constexpr int RW = kOutY / 2;              // rows of a warp
-    __shared__ float P[9 * kOutPlane];         // [tap][kOutY][kOutPitch]
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q = lane & 3;
+__global__ void __launch_bounds__(kOutThreads, out_blocks(CIN)) conv_out_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                                  const __nv_bfloat16* __restrict__ w, float b,
+                                                                                  const float* __restrict__ vol,
+                                                                                  float* __restrict__ out, int D, int H, int W,
+                                                                                  int tx, int ty, int zc) {
+    constexpr int NG = CIN / 8, PL = out_plane();
+    extern __shared__ __align__(16) uint4 out_sm[];   // two slices of NG planes, then the weights
+    float4* sw = reinterpret_cast<float4*>(out_sm + 2 * NG * PL);   // [dy, dx][c]: dz = 0, 1, 2
+    const int tid = threadIdx.x, xg = tid % (kOutX / kOutV), row = tid / (kOutX / kOutV);
     const int bx = (int)(blockIdx.x % (unsigned)tx), bt = (int)(blockIdx.x / (unsigned)tx);
-    const int x0 = bx * kOutX, y0 = bt % ty * kOutY, z0 = bt / ty * kOutZ, zend = min(z0 + kOutZ, D);
-    uint32_t wb[KS][3][2][2];                  // [step][dy][column tile][K half]
-#pragma unroll
-    for (int k = 0; k < KS; ++k)
-#pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                const int n = 8 * t + g, tap = n < 9 ? (n / 3 * 3 + dy) * 3 + n % 3 : 0;
-                const __nv_bfloat16* src = w + tap * CIN + 16 * k + CQ * q;
-                wb[k][dy][t][0] = n < 9 ? pack_bf16(src[0], src[1]) : 0u;
-                wb[k][dy][t][1] = n < 9 && CQ == 4 ? pack_bf16(src[CQ - 2], src[CQ - 1]) : 0u;
-            }
-    // the thread's two output voxels and their sums for slices s - 1, s, s + 1 (s: input slice)
-    const int ox = tid & 63, oy = tid >> 6;    // rows oy and oy + 4
-    float o0[2] = {0.f, 0.f}, o1[2] = {0.f, 0.f}, o2[2];
-    const int xb = (wid & 3) * 16, rb = (wid >> 2) * RW;
-    for (int s = max(z0 - 1, 0); s <= min(zend, D - 1); ++s) {
-        uint32_t a[RW + 2][KS][2][2];          // [input row rb - 1 + j][step][voxel g / g + 8][K half]
-#pragma unroll
-        for (int j = 0; j < RW + 2; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int gy = y0 + rb + j - 1, gx = x0 + xb + g + 8 * h - 1;
-                const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
-                const __nv_bfloat16* src = x + (((long)s * H + (ok ? gy : 0)) * W + (ok ? gx : 0)) * CIN + CQ * q;
-#pragma unroll
-                for (int k = 0; k < KS; ++k) {
-                    if constexpr (CQ == 4) {
-                        const uint2 v = ok ? __ldg(reinterpret_cast<const uint2*>(src + 16 * k)) : make_uint2(0u, 0u);
-                        a[j][k][h][0] = v.x;
-                        a[j][k][h][1] = v.y;
-                    } else {
-                        a[j][k][h][0] = ok ? __ldg(reinterpret_cast<const uint32_t*>(src)) : 0u;
-                        a[j][k][h][1] = 0u;
-                    }
-                }
-            }
-#pragma unroll
-        for (int r = 0; r < RW; ++r)
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-                    for (int k = 0; k < KS; ++k) {
-                        const uint32_t(&f)[2][2] = a[r + dy][k];
-                        mma_bf16(c, f[0][0], f[1][0], f[0][1], f[1][1], wb[k][dy][t][0], wb[k][dy][t][1]);
-                    }
-                float* d = P + (8 * t + 2 * q) * kOutPlane + (rb + r) * kOutPitch + xb + g;
-                if (t == 0 || q == 0) {        // column 8 is the last
-                    d[0] = c[0];
-                    d[8] = c[2];
-                }
-                if (t == 0) {
-                    d[kOutPlane] = c[1];
-                    d[kOutPlane + 8] = c[3];
-                }
-            }
-        __syncthreads();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            o2[h] = 0.f;
-            if (ox < kOutX) {
-                float sum[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-                for (int t = 0; t < 9; ++t) sum[t / 3] += P[t * kOutPlane + (oy + 4 * h) * kOutPitch + ox + t % 3];
-                o0[h] += sum[2];   // dz = 2: input slice s is z + 1 of output slice s - 1
-                o1[h] += sum[1];
-                o2[h] = sum[0];
-                const int gx = x0 + ox, gy = y0 + oy + 4 * h;
-                auto put = [&](int z, float acc) {
-                    const long i = ((long)z * H + gy) * W + gx;
-                    out[i] = __ldg(vol + i) + __bfloat162float(__float2bfloat16(b + acc));
-                };
-                if (gx < W && gy < H) {
-                    if (s - 1 >= z0) put(s - 1, o0[h]);
-                    if (s == D - 1 && s < zend) put(s, o1[h]);   // no slice above the last
-                }
-            }
-            o0[h] = o1[h];
-            o1[h] = o2[h];
+    const int x0 = bx * kOutX, y0 = bt % ty * kOutY, z0 = bt / ty * zc, zend = min(z0 + zc, D);
+    for (int i = tid; i < 9 * CIN; i += kOutThreads)
+        sw[i] = make_float4(__bfloat162float(w[i]), __bfloat162float(w[9 * CIN + i]), __bfloat162float(w[18 * CIN + i]), 0.f);
+    auto stage = [&](int s) {
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(out_sm + (s & 1) * NG * PL);
+        for (int e = tid; e < (kOutY + 2) * (kOutX + 2) * NG; e += kOutThreads) {
+            const int g = e % NG, v = e / NG, px = v % (kOutX + 2), r = v / (kOutX + 2);
+            const int gx = x0 + px - 1, gy = y0 + r - 1;
+            const bool ok = gx >= 0 && gx < W && gy >= 0 && gy < H;
+            const __nv_bfloat16* src = ok ? x + (((long)s * H + gy) * W + gx) * CIN + 8 * g : x;
+            const int at = g * PL + r * kOutRow + px % kOutV * (kOutX / kOutV + 1) + px / kOutV;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(base + 16u * (uint32_t)at), "l"(src),
+                         "r"(ok ? 16 : 0)
+                         : "memory");
         }
-        __syncthreads();   // P is rewritten for the next slice
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    // sums of the output slices s - 1, s and s + 1 (s: input slice)
+    float a0[kOutV], a1[kOutV], a2[kOutV];
+#pragma unroll
+    for (int k = 0; k < kOutV; ++k) a0[k] = a1[k] = b;
+    const int first = max(z0 - 1, 0), last = min(zend, D - 1);
+    stage(first);
+    for (int s = first; s <= last; ++s) {
+        if (s < last) {
+            stage(s + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncthreads();
+        const uint4* in = out_sm + (s & 1) * NG * PL + row * kOutRow + xg;
+#pragma unroll
+        for (int k = 0; k < kOutV; ++k) a2[k] = b;
+#pragma unroll 1
+        for (int dy = 0; dy < 3; ++dy) {
+            uint4 v[kOutV + 2][NG];
+#pragma unroll
+            for (int k = 0; k < kOutV + 2; ++k)
+#pragma unroll
+                for (int g = 0; g < NG; ++g)
+                    v[k][g] = in[g * PL + dy * kOutRow + k % kOutV * (kOutX / kOutV + 1) + k / kOutV];
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+                for (int c = 0; c < CIN; ++c) {
+                    const float4 q = sw[(3 * dy + dx) * CIN + c];
+#pragma unroll
+                    for (int k = 0; k < kOutV; ++k) {
+                        const uint4& u = v[k + dx][c / 8];
+                        const uint32_t h = c % 8 < 2 ? u.x : c % 8 < 4 ? u.y : c % 8 < 6 ? u.z : u.w;
+                        const float f = __uint_as_float(c % 2 ? h & 0xffff0000u : h << 16);
+                        a2[k] = fmaf(q.x, f, a2[k]);
+                        a1[k] = fmaf(q.y, f, a1[k]);
+                        a0[k] = fmaf(q.z, f, a0[k]);
+                    }
+                }
+        }
+        const int gy = y0 + row;
+#pragma unroll
+        for (int k = 0; k < kOutV; ++k) {
+            const int gx = x0 + kOutV * xg + k;
+            auto emit = [&](int z, float acc) {
+                const long i = ((long)z * H + gy) * W + gx;
+                out[i] = vol[i] + __bfloat162float(__float2bfloat16(acc));
+            };
+            if (gx < W && gy < H) {
+                if (s - 1 >= z0) emit(s - 1, a0[k]);
+                if (s == D - 1 && s < zend) emit(s, a1[k]);   // no slice above the last
+            }
+            a0[k] = a1[k];
+            a1[k] = a2[k];
+        }
+        __syncthreads();   // slice s is replaced by s + 2
     }
+}
+
+// Slices per block of a march: the fewest steps over the rounds of resident blocks, where a chunk of zc
+// slices takes zc + extra steps (64^3, last convolution: chunks of 32 slices 95 us, of this rule 29).
+int march_chunk(long tiles, long D, long resident, int extra) {
+    int best = 1;
+    double least = 0.0;
+    for (int zc = 1; zc <= 64; zc += zc < 16 ? 1 : zc / 8) {
+        const long blocks = tiles * ((D + zc - 1) / zc);
+        const double cost = (double)((blocks + 148 * resident - 1) / (148 * resident)) * (zc + extra);
+        if (zc == 1 || cost < least) { least = cost; best = zc; }
+    }
+    return best;
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -395,10 +378,12 @@ int tigre_unet_conv_in(const float* d_vol, const void* d_w, const float* d_b, vo
     cudaStream_t st = (cudaStream_t)stream;
     const __nv_bfloat16* w = (const __nv_bfloat16*)d_w;
     __nv_bfloat16* y = (__nv_bfloat16*)d_y;
-    const long tx = (W + kInX - 1) / kInX, ty = (H + kInY - 1) / kInY, blocks = tx * ty * ((D + kInZ - 1) / kInZ);
+    const long tx = (W + kInX - 1) / kInX, ty = (H + kInY - 1) / kInY;
+    const int zc = march_chunk(tx * ty, D, kInBlocks, 1);
+    const long blocks = tx * ty * ((D + zc - 1) / zc);
     if (blocks > INT_MAX || D > INT_MAX - 64 || H > INT_MAX - 64 || W > INT_MAX - 128)
         return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_in: volume too large");
-    auto go = [&](auto kern) { kern<<<(unsigned)blocks, 256, 0, st>>>(d_vol, w, d_b, y, (int)D, (int)H, (int)W, (int)tx, (int)ty, relu); };
+    auto go = [&](auto kern) { kern<<<(unsigned)blocks, kInThreads, 0, st>>>(d_vol, w, d_b, y, (int)D, (int)H, (int)W, (int)tx, (int)ty, zc, relu); };
     if (Cout == 8) go(conv_in_kernel<8>);
     else if (Cout == 16) go(conv_in_kernel<16>);
     else if (Cout == 32) go(conv_in_kernel<32>);
@@ -414,11 +399,15 @@ int tigre_unet_conv_out(const void* d_x, long Cin, const void* d_w, float b, con
     cudaStream_t st = (cudaStream_t)stream;
     const __nv_bfloat16* x = (const __nv_bfloat16*)d_x;
     const __nv_bfloat16* w = (const __nv_bfloat16*)d_w;
-    const long tx = (W + kOutX - 1) / kOutX, ty = (H + kOutY - 1) / kOutY, blocks = tx * ty * ((D + kOutZ - 1) / kOutZ);
+    const long tx = (W + kOutX - 1) / kOutX, ty = (H + kOutY - 1) / kOutY;
+    const int zc = march_chunk(tx * ty, D, out_blocks((int)Cin), 2);
+    const long blocks = tx * ty * ((D + zc - 1) / zc);
     if (blocks > INT_MAX || D > INT_MAX - 64 || H > INT_MAX - 64 || W > INT_MAX - 128)
         return fail(TIGRE_ERR_BAD_ASSERT, "unet conv_out: volume too large");
     auto go = [&](auto kern) -> int {
-        kern<<<(unsigned)blocks, 256, 0, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W, (int)tx, (int)ty);
+        const int smem = (int)out_smem((int)Cin);
+        TIGRE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kern<<<(unsigned)blocks, kOutThreads, smem, st>>>(x, w, b, d_vol, d_out, (int)D, (int)H, (int)W, (int)tx, (int)ty, zc);
         TIGRE_LAUNCHED();
         return TIGRE_SUCCESS;
     };
