@@ -431,6 +431,7 @@ __global__ void __launch_bounds__(128) conv_fwd_tc_kernel(const __nv_bfloat16* _
     for (int s = 0; s < STAGES; ++s) wait_stage(s);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const long row = m0 + 32 * wid + lane;
+    ok_all = __all_sync(0xffffffffu, ok_all);   // the loads below take whole warps
     if (ok_all) {
 #pragma unroll
         for (int t = 0; t < BN / 16; ++t) {
@@ -470,8 +471,9 @@ __global__ void __launch_bounds__(128) conv_fwd_tc_kernel(const __nv_bfloat16* _
                     reinterpret_cast<uint4*>(yb + o)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
                 }
             }
+            __syncwarp();   // the next load takes the whole warp
         }
-    } else if (tid == 0 && status) {
+    } else if (lane == 0 && status) {
         atomicOr(status, 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_const
     }
     __syncwarp();
     // ---- epilogue: all 4 warps ----
-    const bool done = bar_wait(su32(&done_bar), 0u);
+    const bool done = __all_sync(0xffffffffu, bar_wait(su32(&done_bar), 0u));   // the loads below take whole warps
     __syncthreads();
     if (done && !abort_flag) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -223,32 +223,34 @@ __global__ void __launch_bounds__(128, 1) conv_tc_halo_kernel(const __grid_const
                       "=r"(v[15])
                     : "r"(taddr));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (!inside) continue;
-                float f[16];
+                if (inside) {
+                    float f[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    f[j] = __uint_as_float(v[j]) + (p.bias ? __ldg(p.bias + c0 + j) : 0.f);
-                    if (p.relu) f[j] = fmaxf(f[j], 0.f);
-                }
-                const size_t o = vox * N + c0;
-                if (p.yf) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        reinterpret_cast<float4*>(p.yf + o)[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
-                }
-                if (p.yb) {
-                    uint32_t pk[8];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
-                        pk[q] = *reinterpret_cast<const uint32_t*>(&h);
+                    for (int j = 0; j < 16; ++j) {
+                        f[j] = __uint_as_float(v[j]) + (p.bias ? __ldg(p.bias + c0 + j) : 0.f);
+                        if (p.relu) f[j] = fmaxf(f[j], 0.f);
                     }
-                    reinterpret_cast<uint4*>(p.yb + o)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    reinterpret_cast<uint4*>(p.yb + o)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                    const size_t o = vox * N + c0;
+                    if (p.yf) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            reinterpret_cast<float4*>(p.yf + o)[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+                    }
+                    if (p.yb) {
+                        uint32_t pk[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
+                            pk[q] = *reinterpret_cast<const uint32_t*>(&h);
+                        }
+                        reinterpret_cast<uint4*>(p.yb + o)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                        reinterpret_cast<uint4*>(p.yb + o)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                    }
                 }
+                __syncwarp();   // lanes outside store nothing; the next load takes the whole warp
             }
         }
-    } else if (!done && tid == 0 && p.status) {
+    } else if (!done && lane == 0 && p.status) {
         atomicOr(p.status, TIGRE_STATUS_WAIT_EXPIRED);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
