@@ -334,3 +334,37 @@ def test_first_and_last_convolution_order(c, D, H, W):
         for k in range(c):
             acc = (acc.double() + v[..., k] * wo[t, k].double()).float()
     assert torch.equal(out, vol + acc.bfloat16().float())
+
+
+@pytest.mark.parametrize("D,H,W", [(4, 16, 8), (5, 17, 9)])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (16, 16)])
+def test_convolution_into_any_address(D, H, W, cin, cout):
+    """Outputs that do not start on 16 bytes take the kernels with single-element stores: the same
+    values but for the order of FP32 sums (27 cin terms) and, in BF16, the step to the neighbouring value that
+    it can cause (eight significant bits: 2^-7 of the value at most)."""
+    import torch
+    from tigre_b200 import _native as N
+    g = torch.Generator(device="cuda")
+    g.manual_seed(8)
+    L, p = N.lib(), lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    x = torch.randn((D, H, W, cin), device="cuda", generator=g).bfloat16()
+    w = torch.randn((cout, 27 * cin), device="cuda", generator=g).bfloat16()
+    dy = torch.randn((D, H, W, cout), device="cuda", generator=g).bfloat16()
+    col = torch.empty(2 * 27 * D * H * W * max(cin, cout), dtype=torch.bfloat16, device="cuda")
+    n, ref, got = D * H * W, {}, {}
+    for out, shift in ((ref, 0), (got, 1)):
+        yb = torch.empty(n * cout + shift, dtype=torch.bfloat16, device="cuda")[shift:]
+        yf = torch.empty(n * cout + shift, device="cuda")[shift:]
+        dx = torch.empty(n * cin + shift, device="cuda")[shift:]
+        for y, args in ((yb, (p(yb), None)), (yf, (None, p(yf)))):
+            N.check(L.tigre_conv3d_fwd(p(x), p(w), None, *args, D, H, W, cin, cout, 0, p(col), None), "fwd")
+        N.check(L.tigre_conv3d_bwd_data(p(dy), p(w), p(dx), D, H, W, cin, cout, p(col), None), "bwd_data")
+        out.update(yb=yb.double(), yf=yf.double(), dx=dx.double())
+    size = 27 * max(cin, cout) * float(x.abs().max() * w.abs().max() + dy.abs().max() * w.abs().max())
+    for k, v in ref.items():
+        bar = 2.0 ** -23 * size + (2.0 ** -7 * v.abs() if k == "yb" else 0.0)
+        assert bool(((got[k] - v).abs() <= bar).all()), k
+    half = torch.empty(n * cout + 1, dtype=torch.bfloat16, device="cuda")[1:]
+    rc = L.tigre_conv3d_fwd_pair(p(x), cin // 2, p(x), cin // 2, p(w), None, p(half), D, H, W, cout, 0, p(col), None)
+    assert rc != 0
+

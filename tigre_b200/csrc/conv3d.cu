@@ -560,7 +560,9 @@ int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void
     cudaStream_t st = (cudaStream_t)stream;
     int tc_mode = g_conv_tcgen05.load();
     int* status = conv_status_word();
-    if (tc_mode == 3 && ((uintptr_t)d_x & 15) == 0 && ((uintptr_t)d_col & 15) == 0 &&
+    // the tcgen05 kernels store 16 bytes at a time; the others take any output address
+    const bool y_aligned = (((uintptr_t)d_y_bf16 | (uintptr_t)d_y_f32) & 15) == 0;
+    if (tc_mode == 3 && ((uintptr_t)d_x & 15) == 0 && ((uintptr_t)d_col & 15) == 0 && y_aligned &&
         27L * Cin * Cout <= tigre_conv3d_col_elems(D, H, W, Cin) && conv_tc_halo_supported(D, H, W, Cin, Cout))
         return launch_conv_tc_halo((const __nv_bfloat16*)d_x, nullptr, 0, (const __nv_bfloat16*)d_w, d_bias,
                                    (__nv_bfloat16*)d_y_bf16, d_y_f32, D, H, W, Cin, Cout, relu, 0,
@@ -568,7 +570,7 @@ int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void
     if (tc_mode == 3) tc_mode = 2;
     // the other paths index the im2col matrix (M x 27 Cin) with 32-bit row counts
     if (M * K >= (1L << 31) * 4L || M >= (1L << 31) / 64 * 64) return fail(TIGRE_ERR_BAD_ASSERT, "conv3d too large");
-    const bool tc_wanted = tc_mode == 1 || (tc_mode == 2 && (Cin <= 16 || Cout == 16));
+    const bool tc_wanted = y_aligned && (tc_mode == 1 || (tc_mode == 2 && (Cin <= 16 || Cout == 16)));
     if (tc_wanted && Cin % 8 == 0 && Cout % 16 == 0 && ((uintptr_t)d_x & 15) == 0 && ((uintptr_t)d_w & 15) == 0) {
         // tensor-core (tcgen05) implicit GEMM: N tile = the largest of 128 / 64 / 48 / 32 / 16 dividing Cout
         const __nv_bfloat16* xb = (const __nv_bfloat16*)d_x;
@@ -622,7 +624,7 @@ int tigre_conv3d_fwd_pair(const void* d_xa, long Ca, const void* d_xb, long Cb, 
                           void* d_y_bf16, long D, long H, long W, long Cout, int relu, void* d_col, void* stream) {
     TIGRE_NVTX("tigre_conv3d_fwd_pair");
     if (!d_xa || !d_xb || !d_w || !d_y_bf16 || !d_col) return fail(TIGRE_ERR_BAD_ASSERT, "bad conv3d arguments");
-    if (!tigre_conv3d_fwd_pair_ok(D, H, W, Ca, Cb, Cout) || (((uintptr_t)d_xa | (uintptr_t)d_xb | (uintptr_t)d_col) & 15))
+    if (!tigre_conv3d_fwd_pair_ok(D, H, W, Ca, Cb, Cout) || (((uintptr_t)d_xa | (uintptr_t)d_xb | (uintptr_t)d_y_bf16 | (uintptr_t)d_col) & 15))
         return fail(TIGRE_ERR_BAD_ASSERT, "conv3d of a pair: channels in multiples of 16, 16-byte aligned buffers");
     return launch_conv_tc_halo((const __nv_bfloat16*)d_xa, (const __nv_bfloat16*)d_xb, Cb, (const __nv_bfloat16*)d_w, d_bias,
                                (__nv_bfloat16*)d_y_bf16, nullptr, D, H, W, Ca + Cb, Cout, relu, 0, (__nv_bfloat16*)d_col,
@@ -637,7 +639,7 @@ int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D
         return fail(TIGRE_ERR_BAD_ASSERT, "bad conv3d arguments");
     const long M = D * H * W, K = 27 * Cin;
     cudaStream_t st = (cudaStream_t)stream;
-    if (g_conv_tcgen05.load() == 3 && ((uintptr_t)d_dy & 15) == 0 && ((uintptr_t)d_dcol & 15) == 0 &&
+    if (g_conv_tcgen05.load() == 3 && (((uintptr_t)d_dy | (uintptr_t)d_dx | (uintptr_t)d_dcol) & 15) == 0 &&
         Cout <= 2 * M && conv_tc_halo_supported(D, H, W, Cout, Cin)) {   // d_dcol holds the arranged weights
         // the data gradient is the convolution of dy with the tap-flipped, channel-transposed
         // weights: the halo kernel, FP32 output, no im2col (d_dcol holds the arranged weights)

@@ -309,7 +309,7 @@ static void conv_tc_shape(int N, int D, int nchunks, int* zt, int* stages, uint3
         for (int i = 0; i < 3; ++i) {
             const int z = cand[i];
             // slices past the last one are computed for nothing: at most a quarter of them
-            if ((D + z - 1) / z * z * 4 > 5 * D || (size_t)z * N > 512) continue;
+            if ((D + z - 1L) / z * z * 4 > 5L * D || (size_t)z * N > 512) continue;
             const uint32_t tb = (uint32_t)(kHx * kHy * (z + 2) * kCC * 2), wb = (uint32_t)(27 * kCC * N * 2);
             const uint32_t stb = (tb + wb + 1023u) & ~1023u;
             for (int s = std::min(3, nchunks); s >= 1; --s) {
