@@ -368,3 +368,33 @@ def test_convolution_into_any_address(D, H, W, cin, cout):
     rc = L.tigre_conv3d_fwd_pair(p(x), cin // 2, p(x), cin // 2, p(w), None, p(half), D, H, W, cout, 0, p(col), None)
     assert rc != 0
 
+
+@pytest.mark.parametrize("at", [(-1, -1, -1), (-1, 2, 3), (0, -1, 5), (1, 3, -1), (2, 2, 15)])
+@pytest.mark.parametrize("D,H,W", [(5, 6, 17), (4, 5, 31), (7, 4, 16)])
+def test_weight_gradient_beside_an_infinite_activation(D, H, W, at):
+    """An infinite voxel shows in the taps that use it and in no other."""
+    import torch
+    from tigre_b200 import _native as N
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    cin, cout = 32, 48
+    x = torch.randn((D, H, W, cin), device="cuda", generator=g).bfloat16()
+    dy = torch.randn((D, H, W, cout), device="cuda", generator=g).bfloat16()
+    dy[dy == 0] = 1.0
+    x[at][3] = float("inf")
+    col = torch.empty(27 * D * H * W * cin, dtype=torch.bfloat16, device="cuda")
+    dw = torch.zeros((cout, 27, cin), device="cuda")
+    N.check(N.lib().tigre_conv3d_bwd_weight(C.c_void_p(x.data_ptr()), C.c_void_p(dy.data_ptr()), C.c_void_p(dw.data_ptr()),
+                                            D, H, W, cin, cout, C.c_void_p(col.data_ptr()), None), "bwd_weight")
+    ref = torch.empty((cout, 27, cin), dtype=torch.float64, device="cuda")
+    for t in range(27):      # overlapping parts only: no padding to multiply
+        a, b = [], []
+        for n, o in ((D, t // 9 - 1), (H, t // 3 % 3 - 1), (W, t % 3 - 1)):
+            a.append(slice(max(0, -o), n - max(0, o)))
+            b.append(slice(max(0, o), n + min(0, o)))
+        ref[:, t] = dy[tuple(a)].double().reshape(-1, cout).T @ x[tuple(b)].double().reshape(-1, cin)
+    fine = ref.isfinite()
+    assert not bool(fine.all()) and torch.equal(fine, dw.isfinite())
+    assert torch.equal(ref[~fine], dw[~fine].double())
+    assert float((dw[fine].double() - ref[fine]).norm() / ref[fine].norm()) < 1e-5
+

@@ -123,10 +123,20 @@ __global__ void __launch_bounds__(kWgThreads, 2) conv_wgrad_kernel(WgArgs p) {
         }
         __syncthreads();
         const uint32_t sx = base + (uint32_t)buf * kStage, sd = sx + kXBytes;
+        // Places of the tile past the volume's end hold dy = 0, but x may have a voxel of the volume
+        // beside them, and 0 times an infinite one is no 0: rows of such places are left out, and in the
+        // others their x is cleared (K index 2 (lane % 4) + e of the low half, + 8 of the high one).
+        const long tr = tile / p.tx;
+        const int nx = p.W - (int)(tile % p.tx) * kTX, ny = min(p.H - (int)(tr % p.ty) * kTY, kTY);
+        const int nz = min(p.D - (int)(tr / p.ty) * kTZ, kTZ);
+        const int kx = (lane & 3) * 2;
+        const uint32_t m0 = (kx < nx ? 0xffffu : 0u) | (kx + 1 < nx ? 0xffff0000u : 0u);
+        const uint32_t m1 = (kx + 8 < nx ? 0xffffu : 0u) | (kx + 9 < nx ? 0xffff0000u : 0u);
 #pragma unroll 1
-        for (int z = 0; z < kTZ; ++z) {
+        for (int z = 0; z < nz; ++z) {
 #pragma unroll
             for (int y = 0; y < kTY; ++y) {
+                if (y >= ny) break;
                 uint32_t a[MT][4];
 #pragma unroll
                 for (int m = 0; m < MT; ++m)
@@ -136,6 +146,10 @@ __global__ void __launch_bounds__(kWgThreads, 2) conv_wgrad_kernel(WgArgs p) {
                 for (int t = 0; t < 3; ++t) {
                     uint32_t b[4];
                     ldsm4t(row + (uint32_t)(t * kRowX), b);
+                    b[0] &= m0;
+                    b[1] &= m1;
+                    b[2] &= m0;
+                    b[3] &= m1;
 #pragma unroll
                     for (int m = 0; m < MT; ++m) {
                         mma(acc[t][m][0], a[m], b[0], b[1]);
@@ -236,7 +250,9 @@ __global__ void __launch_bounds__(128) bias_grad_kernel(const float* __restrict_
 
 }  // namespace
 
-bool conv_wgrad_supported(long Cin, long Cout) { return Cin % kCI == 0 && Cout % 16 == 0; }
+bool conv_wgrad_supported(long Cin, long Cout) {
+    return Cin % kCI == 0 && Cout % 16 == 0 && (Cin / kCI) * (Cout / 16) <= 65535;   // one block row per channel tile
+}
 
 int launch_conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw, long D, long H, long W, long Cin,
                       long Cout, float* work, cudaStream_t st) {
