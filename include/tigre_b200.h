@@ -302,6 +302,11 @@ int tigre_philox4x32(unsigned int* d_out, long long nblocks, unsigned long long 
  * channel minor), zero padding 1, FP32 accumulation on the tensor cores.  d_col: scratch of
  * tigre_conv3d_col_elems(D, H, W, Cin) BF16 elements (d_dcol: as many floats). */
 long long tigre_conv3d_col_elems(long D, long H, long W, long C);
+/* BF16 elements that tigre_conv3d_fwd and tigre_conv3d_bwd_weight use of d_col, at most
+ * tigre_conv3d_col_elems, when d_col and all inputs start on 16 bytes (w too).  A buffer serves one call
+ * at a time: calls that may overlap, on other streams or from other threads, need their own. */
+long long tigre_conv3d_fwd_work(long D, long H, long W, long Cin, long Cout);
+long long tigre_conv3d_bwd_weight_work(long D, long H, long W, long Cin, long Cout);
 /* Forward path of tigre_conv3d_fwd (and of the data gradient): 3 (default) the tcgen05 halo-tile
  * kernel -- one TMA load of a zero-padded input tile per 16 input channels, the 27 taps as
  * shifted shared-memory operand descriptors, TMEM accumulators -- wherever Cin % 16 == 0 and
@@ -316,7 +321,8 @@ int tigre_conv3d_set_tcgen05(int mode);
 int tigre_conv3d_status(int reset);
 int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void* d_y_bf16, float* d_y_f32, long D,
                      long H, long W, long Cin, long Cout, int relu, void* d_col, void* stream);
-/* y (BF16) = conv of the channel concatenation [xa (Ca), xb (Cb)], each read where it is.
+/* y (BF16) = conv of the channel concatenation [xa (Ca), xb (Cb)], each read where it is; d_col:
+ * 27 (Ca + Cb) Cout BF16 elements, all buffers but the weights and the bias on 16 bytes.
  * tigre_conv3d_fwd_pair_ok: 1 where this form runs (multiples of 16 channels, forward path 3). */
 int tigre_conv3d_fwd_pair_ok(long D, long H, long W, long Ca, long Cb, long Cout);
 int tigre_conv3d_fwd_pair(const void* d_xa, long Ca, const void* d_xb, long Cb, const void* d_w, const float* d_bias,

@@ -398,3 +398,69 @@ def test_weight_gradient_beside_an_infinite_activation(D, H, W, at):
     assert torch.equal(ref[~fine], dw[~fine].double())
     assert float((dw[fine].double() - ref[fine]).norm() / ref[fine].norm()) < 1e-5
 
+
+@pytest.mark.parametrize("threads", [False, True])
+def test_convolutions_that_overlap(threads):
+    """Training steps of four layers at once, each on a stream of its own from one thread or on one stream from a
+    thread each, give what they give one after the other."""
+    import threading
+    import torch
+    from tigre_b200 import warmstart
+    g = torch.Generator(device="cuda")
+    g.manual_seed(10)
+    layers = []
+    for cin, cout in ((16, 32), (32, 32), (64, 16), (48, 64)):
+        x = torch.randn((20, 17, 24, cin), device="cuda", generator=g).bfloat16()
+        w = torch.randn((cout, 27 * cin), device="cuda", generator=g) * 0.05
+        dy = torch.randn((20, 17, 24, cout), device="cuda", generator=g).bfloat16()
+        layers.append((x, w, torch.zeros(cout, device="cuda"), dy))
+
+    def step(layer):
+        x, w, b = (t.detach().requires_grad_(True) for t in layer[:3])
+        y = warmstart.conv3d(x, w, b, True)
+        y.backward(layer[3])
+        return [y.detach(), x.grad, w.grad, b.grad]
+    want = [step(layer) for layer in layers]
+    torch.cuda.synchronize()
+    got = [[] for _ in layers]
+    if threads:
+        def work(i):
+            got[i].extend(step(layers[i]) for _ in range(15))
+        ts = [threading.Thread(target=work, args=(i,)) for i in range(len(layers))]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+    else:
+        streams = [torch.cuda.Stream() for _ in layers]
+        for _ in range(15):
+            for i, st in enumerate(streams):
+                with torch.cuda.stream(st):
+                    got[i].append(step(layers[i]))
+    torch.cuda.synchronize()
+    for i, outs in enumerate(got):
+        assert len(outs) == 15
+        for o in outs:
+            assert all(torch.equal(a, b) for a, b in zip(o, want[i])), i
+
+
+@pytest.mark.parametrize("D,H,W,cin,cout", [(5, 6, 7, 16, 32), (4, 16, 8, 32, 32), (1, 1, 1, 16, 16), (6, 5, 4, 24, 40),
+                                            (3, 4, 5, 5, 6), (9, 8, 7, 48, 64)])
+def test_convolution_scratch_of_the_stated_size(D, H, W, cin, cout):
+    """The calls stay inside the elements that the size queries state, and those inside the im2col matrix."""
+    import torch
+    from tigre_b200 import _native as N
+    L, p = N.lib(), lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    x = torch.ones((D, H, W, cin), device="cuda").bfloat16()
+    w = torch.ones((cout, 27 * cin), device="cuda").bfloat16()
+    dy = torch.ones((D, H, W, cout), device="cuda").bfloat16()
+    y, dw = torch.empty_like(dy), torch.zeros((cout, 27 * cin), device="cuda")
+    full = int(L.tigre_conv3d_col_elems(D, H, W, cin))
+    fwd, bwd = (int(f(D, H, W, cin, cout)) for f in (L.tigre_conv3d_fwd_work, L.tigre_conv3d_bwd_weight_work))
+    assert 0 < fwd <= full and 0 < bwd <= full
+    for n, call in ((fwd, lambda c: L.tigre_conv3d_fwd(p(x), p(w), None, p(y), None, D, H, W, cin, cout, 0, c, None)),
+                    (bwd, lambda c: L.tigre_conv3d_bwd_weight(p(x), p(dy), p(dw), D, H, W, cin, cout, c, None))):
+        col = torch.full((full + 64,), 7.0, device="cuda").bfloat16()      # what lies behind stays
+        N.check(call(p(col)), "conv3d")
+        assert bool((col[n:] == 7.0).all())
+

@@ -127,6 +127,8 @@ _SIGS = {
                                       C.c_long, C.c_long, C.c_void_p]),
     "tigre_conv3d_fwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_long, C.c_long,
                                    C.c_long, C.c_long, C.c_long, C.c_int, C.c_void_p, C.c_void_p]),
+    "tigre_conv3d_fwd_work": (C.c_longlong, [C.c_long] * 5),
+    "tigre_conv3d_bwd_weight_work": (C.c_longlong, [C.c_long] * 5),
     "tigre_conv3d_fwd_pair_ok": (C.c_int, [C.c_long] * 6),
     "tigre_conv3d_fwd_pair": (C.c_int, [C.c_void_p, C.c_long, C.c_void_p, C.c_long, C.c_void_p, C.c_void_p, C.c_void_p,
                                         C.c_long, C.c_long, C.c_long, C.c_long, C.c_int, C.c_void_p, C.c_void_p]),

@@ -551,6 +551,21 @@ int tigre_conv3d_status(int reset) {
 
 long long tigre_conv3d_col_elems(long D, long H, long W, long C) { return 27LL * D * H * W * C; }
 
+// What the path that runs touches of the scratch.  The halo-tile kernel keeps its arranged weights there and
+// the implicit GEMMs nothing, whichever mode is set meanwhile; the other layers write the im2col matrix.
+long long tigre_conv3d_fwd_work(long D, long H, long W, long Cin, long Cout) {
+    if (D <= 0 || H <= 0 || W <= 0 || Cin <= 0 || Cout <= 0) return 0;
+    const long long full = tigre_conv3d_col_elems(D, H, W, Cin);
+    return Cin % 8 == 0 ? std::min(full, 27LL * Cin * Cout) : full;
+}
+
+long long tigre_conv3d_bwd_weight_work(long D, long H, long W, long Cin, long Cout) {
+    if (D <= 0 || H <= 0 || W <= 0 || Cin <= 0 || Cout <= 0) return 0;
+    if (!conv_wgrad_supported(Cin, Cout) || D >= INT_MAX || H >= INT_MAX || W >= INT_MAX)
+        return tigre_conv3d_col_elems(D, H, W, Cin);
+    return std::max(8L, 2 * conv_wgrad_work(D, H, W, Cin, Cout));
+}
+
 int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void* d_y_bf16, float* d_y_f32, long D,
                      long H, long W, long Cin, long Cout, int relu, void* d_col, void* stream) {
     TIGRE_NVTX("tigre_conv3d_fwd");

@@ -254,6 +254,26 @@ bool conv_wgrad_supported(long Cin, long Cout) {
     return Cin % kCI == 0 && Cout % 16 == 0 && (Cin / kCI) * (Cout / 16) <= 65535;   // one block row per channel tile
 }
 
+// Slices: whole rounds of the 296 resident blocks, at most 256 tiles (2^16 voxels) summed in one
+// accumulator.  They live in the caller's im2col scratch (27 Cin D H W BF16 elements), which
+// holds them (*fits) for all but the smallest volumes; those allocate.
+static long wgrad_splits(long D, long H, long W, long Cin, long Cout, bool* fits) {
+    const long ntiles = ((W + kTX - 1) / kTX) * ((H + kTY - 1) / kTY) * ((D + kTZ - 1) / kTZ);
+    const long chan = Cin / kCI * (Cout / (Cout % 32 == 0 ? 32 : 16)), per = Cout * 27 * Cin;
+    const long round = std::max(1L, 296 / chan);
+    long splits = round * std::max(1L, (ntiles / round + 255) / 256);
+    const long room = 27 * Cin * D * H * W / 2 / per;
+    splits = std::max(1L, std::min(splits, ntiles));
+    *fits = room >= 1;
+    return *fits ? std::min(splits, room) : splits;
+}
+
+long conv_wgrad_work(long D, long H, long W, long Cin, long Cout) {
+    bool fits;
+    const long splits = wgrad_splits(D, H, W, Cin, Cout, &fits);
+    return fits ? splits * Cout * 27 * Cin : 0;
+}
+
 int launch_conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw, long D, long H, long W, long Cin,
                       long Cout, float* work, cudaStream_t st) {
     WgArgs a{};
@@ -266,17 +286,11 @@ int launch_conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw
     a.nci = (int)(Cin / kCI);
     const int CO = Cout % 32 == 0 ? 32 : 16;
     const long chan = a.nci * (Cout / CO), per = Cout * 27 * Cin;
-    // Slices: whole rounds of the 296 resident blocks, at most 256 tiles (2^16 voxels) summed in one
-    // accumulator.  They live in the caller's im2col scratch (27 Cin D H W BF16 elements), which
-    // holds them for all but the smallest volumes; those allocate.
-    const long round = std::max(1L, 296 / chan);
-    long splits = round * std::max(1L, (a.ntiles / round + 255) / 256);
-    const long room = 27 * Cin * D * H * W / 2 / per;
-    splits = std::max(1L, std::min(splits, a.ntiles));
-    if (room >= 1) splits = std::min(splits, room);
+    bool fits;
+    const long splits = wgrad_splits(D, H, W, Cin, Cout, &fits);
     a.splits = (int)splits;
     float* own = nullptr;
-    if (room < 1) TIGRE_CUDA(cudaMallocAsync(&own, sizeof(float) * (size_t)(splits * per), st));
+    if (!fits) TIGRE_CUDA(cudaMallocAsync(&own, sizeof(float) * (size_t)(splits * per), st));
     float* ws = own ? own : work;
     a.ws = ws;
     const dim3 grid((unsigned)splits, (unsigned)chan);

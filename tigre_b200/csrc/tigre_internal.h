@@ -185,6 +185,7 @@ int launch_conv_tc_halo(const __nv_bfloat16* x, const __nv_bfloat16* xb, long Cb
                         float* yf, long D, long H, long W, long Cin, long Cout, int relu, int flip,
                         __nv_bfloat16* wk_scratch, int* status, cudaStream_t st);
 bool conv_wgrad_supported(long Cin, long Cout);
+long conv_wgrad_work(long D, long H, long W, long Cin, long Cout);   // floats of its scratch
 int launch_conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw, long D, long H, long W, long Cin,
                       long Cout, float* work, cudaStream_t st);
 int launch_backproject(TigrePlan* p, const void* proj_pad, int pdt, void* vol, int vdt, int matched, int a0, int a1,

@@ -48,25 +48,13 @@ def _stream(t):
     return s(t)
 
 
-class _Scratch:
-    """Grow-only device scratch for im2col (BF16) and its gradient (FP32)."""
-
-    def __init__(self):
-        self.col = None
-        self.dcol = None
-
-    def get(self, n, kind, device):
-        T = _torch()
-        if kind == "col":
-            if self.col is None or self.col.numel() < n or self.col.device != device:
-                self.col = T.empty(n, dtype=T.bfloat16, device=device)
-            return self.col
-        if self.dcol is None or self.dcol.numel() < n or self.dcol.device != device:
-            self.dcol = T.empty(n, dtype=T.float32, device=device)
-        return self.dcol
-
-
-_SCRATCH = _Scratch()
+def _col(work, sizes, *inputs):
+    """Elements of scratch of a convolution call: work(*sizes) where its inputs start on 16 bytes, else the im2col
+    matrix.  Every call allocates its own from its stream's allocator: calls on other streams or from other
+    threads cannot meet in it."""
+    if any(t.data_ptr() % 16 for t in inputs):
+        work, sizes = N.lib().tigre_conv3d_col_elems, sizes[:4]
+    return work(*sizes)
 
 
 def conv3d(x, w, b, relu):
@@ -86,7 +74,8 @@ def _conv_fn():
             x = x.contiguous()
             wb = w.to(T.bfloat16).contiguous()
             y = T.empty((D, H, W, Cout), dtype=T.bfloat16, device=x.device)
-            col = _SCRATCH.get(int(N.lib().tigre_conv3d_col_elems(D, H, W, Cin)), "col", x.device)
+            col = T.empty(_col(N.lib().tigre_conv3d_fwd_work, (D, H, W, Cin, Cout), x, wb), dtype=T.bfloat16,
+                          device=x.device)
             N.check(N.lib().tigre_conv3d_fwd(C.c_void_p(x.data_ptr()), C.c_void_p(wb.data_ptr()),
                                              C.c_void_p(b.data_ptr()), C.c_void_p(y.data_ptr()), None, D, H, W, Cin,
                                              Cout, 1 if relu else 0, C.c_void_p(col.data_ptr()), _stream(x)),
@@ -100,41 +89,44 @@ def _conv_fn():
             x, wb, y = ctx.saved_tensors
             D, H, W, Cin = x.shape
             Cout = wb.shape[0]
-            if dy.dtype == T.bfloat16 and Cout % 8 == 0 and Cout <= 2048 and dy.contiguous().data_ptr() % 16 == 0:
+            L = N.lib()
+            fused = dy.dtype == T.bfloat16 and Cout % 8 == 0 and Cout <= 2048 and dy.contiguous().data_ptr() % 16 == 0
+            # one scratch for the three steps, which run one after the other (the other inputs of the two
+            # convolutions are allocated here, on 16 bytes)
+            col = T.empty(max(_col(L.tigre_conv3d_bwd_weight_work, (D, H, W, Cin, Cout), x),
+                              L.tigre_conv3d_fwd_work(D, H, W, Cout, Cin) if Cout % 8 == 0 else 0,
+                              2 * L.tigre_conv3d_relu_grad_work(D * H * W, Cout) if fused else 0),
+                          dtype=T.bfloat16, device=x.device)
+            if fused:
                 # ReLU mask and bias sums in one pass
                 dy = dy.contiguous()
                 gb = T.empty_like(dy) if ctx.relu else dy
                 db = T.empty(Cout, dtype=T.float32, device=x.device)
-                work = T.empty(int(N.lib().tigre_conv3d_relu_grad_work(D * H * W, Cout)), dtype=T.float32,
-                               device=x.device)
-                N.check(N.lib().tigre_conv3d_relu_grad(C.c_void_p(dy.data_ptr()), C.c_void_p(y.data_ptr()),
-                                                       C.c_void_p(gb.data_ptr()), C.c_void_p(db.data_ptr()), D * H * W,
-                                                       Cout, 1 if ctx.relu else 0, C.c_void_p(work.data_ptr()),
-                                                       _stream(x)), "tigre_conv3d_relu_grad")
+                N.check(L.tigre_conv3d_relu_grad(C.c_void_p(dy.data_ptr()), C.c_void_p(y.data_ptr()),
+                                                 C.c_void_p(gb.data_ptr()), C.c_void_p(db.data_ptr()), D * H * W,
+                                                 Cout, 1 if ctx.relu else 0, C.c_void_p(col.data_ptr()),
+                                                 _stream(x)), "tigre_conv3d_relu_grad")
             else:
                 g = dy.float()
                 if ctx.relu:
                     g = g * (y > 0)
                 db = g.sum(dim=(0, 1, 2))
                 gb = g.to(T.bfloat16).contiguous()
-            L = N.lib()
             if Cout % 8 == 0:
                 dx = T.empty((D, H, W, Cin), dtype=T.bfloat16, device=x.device)
                 # the data gradient is the forward convolution of dy with the tap-flipped,
                 # channel-transposed weights: wt[c][t*Cout + co] = w[co][(26 - t)*Cin + c]
                 wt = wb.view(Cout, 27, Cin).flip(1).permute(2, 1, 0).reshape(Cin, 27 * Cout).contiguous()
-                col = _SCRATCH.get(int(L.tigre_conv3d_col_elems(D, H, W, Cout)), "col", x.device)
                 N.check(L.tigre_conv3d_fwd(C.c_void_p(gb.data_ptr()), C.c_void_p(wt.data_ptr()), None,
                                            C.c_void_p(dx.data_ptr()), None, D, H, W, Cout, Cin, 0,
                                            C.c_void_p(col.data_ptr()), _stream(x)), "tigre_conv3d_fwd")
             else:
                 dx = T.empty((D, H, W, Cin), dtype=T.float32, device=x.device)
-                dcol = _SCRATCH.get(int(L.tigre_conv3d_col_elems(D, H, W, Cin)), "dcol", x.device)
+                dcol = T.empty(int(L.tigre_conv3d_col_elems(D, H, W, Cin)), dtype=T.float32, device=x.device)
                 N.check(L.tigre_conv3d_bwd_data(C.c_void_p(gb.data_ptr()), C.c_void_p(wb.data_ptr()),
                                                 C.c_void_p(dx.data_ptr()), D, H, W, Cin, Cout,
                                                 C.c_void_p(dcol.data_ptr()), _stream(x)), "tigre_conv3d_bwd_data")
             dw = T.zeros((Cout, 27 * Cin), dtype=T.float32, device=x.device)
-            col = _SCRATCH.get(int(L.tigre_conv3d_col_elems(D, H, W, Cin)), "col", x.device)
             N.check(L.tigre_conv3d_bwd_weight(C.c_void_p(x.data_ptr()), C.c_void_p(gb.data_ptr()),
                                               C.c_void_p(dw.data_ptr()), D, H, W, Cin, Cout,
                                               C.c_void_p(col.data_ptr()), _stream(x)), "tigre_conv3d_bwd_weight")
@@ -230,8 +222,9 @@ def _make_unet_class():
                 d, h, w, cin = x.shape
                 cout = layer.w.shape[0]
                 y = T.empty((d, h, w, cout), dtype=T.bfloat16, device=x.device)
-                col = _SCRATCH.get(int(L.tigre_conv3d_col_elems(d, h, w, cin)), "col", x.device)
-                N.check(L.tigre_conv3d_fwd(p(x), p(self._wbf(layer)), p(layer.b), p(y), None, d, h, w, cin, cout,
+                wb = self._wbf(layer)
+                col = T.empty(_col(L.tigre_conv3d_fwd_work, (d, h, w, cin, cout), x, wb), dtype=T.bfloat16, device=x.device)
+                N.check(L.tigre_conv3d_fwd(p(x), p(wb), p(layer.b), p(y), None, d, h, w, cin, cout,
                                            1 if layer.relu else 0, p(col), st), "tigre_conv3d_fwd")
                 return y
 
@@ -255,7 +248,7 @@ def _make_unet_class():
                     up = T.empty((d, h, w, cx), dtype=T.bfloat16, device=x.device)
                     N.check(L.tigre_unet_up2(p(x), p(up), d, h, w, cx, st), "tigre_unet_up2")
                     y = T.empty((d, h, w, co), dtype=T.bfloat16, device=x.device)
-                    col = _SCRATCH.get(27 * (cx + cs) * co, "col", x.device)
+                    col = T.empty(27 * (cx + cs) * co, dtype=T.bfloat16, device=x.device)
                     N.check(L.tigre_conv3d_fwd_pair(p(up), cx, p(s), cs, p(self._wbf(ca)), p(ca.b), p(y), d, h, w, co,
                                                     1 if ca.relu else 0, p(col), st), "tigre_conv3d_fwd_pair")
                     x = conv(y, cb)
