@@ -90,7 +90,9 @@ def _conv_fn():
             D, H, W, Cin = x.shape
             Cout = wb.shape[0]
             L = N.lib()
-            fused = dy.dtype == T.bfloat16 and Cout % 8 == 0 and Cout <= 2048 and dy.contiguous().data_ptr() % 16 == 0
+            # the fused pass reads 16 bytes at a time; y may be what a saved-tensor hook made of it
+            fused = dy.dtype == T.bfloat16 and Cout % 8 == 0 and Cout <= 2048 and dy.contiguous().data_ptr() % 16 == 0 \
+                and not (ctx.relu and (y.dtype != T.bfloat16 or not y.is_contiguous() or y.data_ptr() % 16))
             # one scratch for the three steps, which run one after the other (the other inputs of the two
             # convolutions are allocated here, on 16 bytes)
             col = T.empty(max(_col(L.tigre_conv3d_bwd_weight_work, (D, H, W, Cin, Cout), x),
