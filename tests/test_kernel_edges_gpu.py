@@ -207,6 +207,32 @@ def test_denoise_in_one_pass_per_iteration(shape, iters):
     assert rc == 4 and "work space" in N.last_error()
 
 
+@pytest.mark.parametrize("room", [6.0, 8.5, 9.0])
+def test_denoise_where_memory_is_short(room, monkeypatch):
+    """The result and five floats per voxel of work space always did; the larger work space is taken only
+    where the result fits beside it."""
+    import torch
+    from tigre_b200.utilities.im_3d_denoise import tv_denoise_device
+    x = torch.from_numpy(np.random.default_rng(8).random((20, 24, 30), dtype=np.float32)).cuda()
+    want = tv_denoise_device(x, 5, 5.0)
+    left = [room * 22 / 20 * x.numel()]      # of the padded volume
+    alloc = {k: getattr(torch, k) for k in ("empty", "empty_like")}
+
+    def short(name):
+        def f(a, *args, **kw):
+            n = a.numel() if torch.is_tensor(a) else int(np.prod(a))
+            if n > left[0]:
+                raise torch.OutOfMemoryError("CUDA out of memory (the test's)")
+            left[0] -= n
+            return alloc[name](a, *args, **kw)
+        return f
+    for k in alloc:
+        monkeypatch.setattr(torch, k, short(k))
+    got = tv_denoise_device(x, 5, 5.0)
+    monkeypatch.undo()
+    _close(got.cpu().numpy(), want.cpu().numpy(), 1e-6)
+
+
 # ---------------------------------------------------------------------------- convolutions --
 def _conv64(x, w, cout):
     import torch

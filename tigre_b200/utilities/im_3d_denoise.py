@@ -38,13 +38,13 @@ def tv_denoise_device(img, niter, lmbda, work=None):
     nz, ny, nx = x.shape
     L = N.lib()
     need = int(L.tigre_tv_denoise_work_floats(nx, ny, nz))
+    out = torch.empty_like(x)     # before the work space, which takes the larger size only where it fits beside it
     if work is None or work.numel() < need:
         # one pass per iteration where its larger work space fits, else two
         try:
             work = torch.empty(int(L.tigre_tv_denoise_fused_floats(nx, ny, nz)), dtype=torch.float32, device=x.device)
         except torch.OutOfMemoryError:
             work = torch.empty(need, dtype=torch.float32, device=x.device)
-    out = torch.empty_like(x)
     spacing = (C.c_float * 3)(1.0, 1.0, 1.0)
     N.check(L.tigre_tv_denoise_ex(C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr()), nx, ny, nz, float(lmbda),
                                   C.cast(spacing, C.c_void_p), int(niter), C.c_void_p(work.data_ptr()),
