@@ -89,6 +89,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
     return false;
 }
 
+// A tap of the patch.  The compiler may order it freely among the arithmetic; that it stays between the wait for
+// the view's copy and the barrier behind which the patch is rewritten is seen to there: its address comes from
+// a value made after the wait, and the sums are asked for before the barrier (volatile loads that
+// clobber memory instead: 0.7 % on 181 x 203 x 190 tilted).
 __device__ __forceinline__ float lds(uint32_t a) {
     float v;
     asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
@@ -240,7 +244,8 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
         // after one expired wait this thread waits no more (its sums are not written)
         if (failed_at < 0 && !mbar_wait(bar, (uint32_t)((i >> 1) & 1))) failed_at = i;
         const float* patch = s ? buf1 : buf0;
-        const uint32_t patch_u32 = s ? buf1_u32 : buf0_u32;
+        uint32_t patch_u32 = s ? buf1_u32 : buf0_u32;
+        asm volatile("" : "+r"(patch_u32) : : "memory");           // lds: no tap before here
         const int u0 = info[s][0], v0 = info[s][1], fits = info[s][2];
         if (active) {
             const FrameBPK& F = p.frames[p.a0 + la];
@@ -455,6 +460,8 @@ __global__ void __launch_bounds__(TXY* TXY, 2) bp_tma_kernel(const __grid_consta
                 }
             }
         }
+#pragma unroll
+        for (int k = 0; k < VZ; ++k) asm volatile("" : : "f"(acc[k]) : "memory");   // lds: no tap behind here
         __syncthreads();   // everyone is done with buffer s
         if (tid < 32 && i + 2 < nviews) plan_patch(p, &tmap, la + 2, x0, y0, z0, s ? buf1 : buf0, bar, info[s], failed_at >= 0);
     }
