@@ -541,24 +541,25 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 // Blocks per tile, a power of two up to 8 (the portable cluster size), from the time that the
-// waves of resident blocks take: a view costs a block 3.8 us when two blocks share an SM and
-// 2.5 us alone (matched, 512^3 and 64^3), and a block 3 us to start and finish, about 8 us
-// with the exchange of the sums.  Sharing is taken where it saves 5 % in this account.  Matched,
-// one block per tile -> shared: 64^3 with 100 views 249 -> 62 us (8 blocks), 96^3 / 60 154 -> 106,
-// 128^3 / 180 445 -> 381, 160^3 / 90 547 -> 437; from 200^3 on the waves fill the chip by
-// themselves (200^3 / 90 measured 890 us alone and 904 us shared).
-int bp_splits(long blocks, int na) {
+// rounds of resident blocks take, as measured over 15 volumes of 16^3 to 200^3, 4 to 180 views and each
+// number of blocks: a view costs a block 2.4 us alone on an SM and 3.9 when two share it (matched; FDK 2.5 and
+// 3.45), the call 6 us beside the views, 13 with the exchange of the sums, and a further round 6.  Sharing is
+// taken from four views a block on and where it saves 5 % in this account (9 % for the eighth
+// block, whose clusters pack worse).  Over the 330 entries no choice is more than 1 % slower than one
+// block a tile.  Matched, one block -> chosen: 64^3 with 100 views 247 -> 63 us (8 blocks), with 16 46 -> 20 (4),
+// 96^3 / 60 153 -> 106 (4), 128^3 / 180 441 -> 381 (2) and / 12 38 (1; two blocks 40), 160^3 / 100 608 -> 471 (4).
+int bp_splits(long blocks, int na, bool matched) {
     constexpr long kSms = 148, kSlots = 2 * kSms;
+    const double alone = matched ? 2.4 : 2.5, shared = matched ? 3.9 : 3.45;
     int best = 1;
     double best_t = 0.0;
     for (int s = 1; s <= kMaxSplit; s *= 2) {
         if (s > 1 && na < 4 * s) break;
         const int views = (na + s - 1) / s;
         const long full = blocks * s / kSlots, rest = blocks * s % kSlots;
-        const double fixed = s == 1 ? 3.0 : 8.0;
-        double t = (double)full * (3.8 * views + fixed);
-        if (rest) t += (rest > kSms ? 3.8 : 2.5) * views + fixed;
-        if (s == 1 || t < 0.95 * best_t) { best = s; best_t = t; }
+        double t = (s == 1 ? 6.0 : 13.0) + 6.0 * (double)(full + (rest > 0) - 1) + (double)full * shared * views;
+        if (rest) t += (rest > kSms ? shared : alone) * views;
+        if (s == 1 || t < (s == 8 ? 0.91 : 0.95) * best_t) { best = s; best_t = t; }
     }
     return best;
 }
@@ -566,7 +567,7 @@ int bp_splits(long blocks, int na) {
 template <typename TV>
 int launch_typed(const CUtensorMap& tm, BPKArgs a, bool matched, bool axial, cudaStream_t st) {
     dim3 grid((a.nX + TXY - 1) / TXY, (a.nY + TXY - 1) / TXY, (a.nZ + VZ - 1) / VZ);
-    a.nsplit = bp_splits((long)grid.x * grid.y * grid.z, a.na);
+    a.nsplit = bp_splits((long)grid.x * grid.y * grid.z, a.na, matched);
     size_t smem = 2 * (((size_t)a.BU * a.BV * sizeof(float) + 127) / 128 * 128) + 128;
     auto go = [&](auto kern) -> int {
         TIGRE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
