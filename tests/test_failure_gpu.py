@@ -5,8 +5,10 @@ TIGRE_OPT_BP_SKIP_COPY makes the TMA-staged backprojector issue no copy (and no 
 one view of each launch, so every block's bounded mbarrier wait for that view runs out with
 nothing in flight.  The threads then wait no more, no further copy is issued, thread 0
 waits for the copy of the next view that was already issued, and the block writes nothing,
-sets TIGRE_STATUS_WAIT_EXPIRED in the plan status word and exits;
-the device call returns normally (the status is the report), the host call returns
+sets TIGRE_STATUS_WAIT_EXPIRED in the plan status word and exits.  Where the blocks of a cluster
+share a tile's views (12 views of 64^3: two blocks), the one that owns the view gives its failure
+to the others with its sums, and none of them writes; with 7 views a block owns its tile alone.
+The device call returns normally (the status is the report), the host call returns
 TIGRE_ERR_CUDA.  Afterwards the same plan and the host entry points give correct results.
 """
 import numpy as np
@@ -45,6 +47,34 @@ def test_expired_wait_sets_status_on_the_device_api(view):
     mx, l2 = G.rel_err(got, O.atb(proj, geo, ang, "matched"))
     assert mx <= TOL and l2 <= TOL, (mx, l2)
     assert plan.status() == 0
+
+
+@pytest.mark.parametrize("views,view", [(12, 0), (12, 5), (12, 6), (12, 11), (7, 0), (7, 3), (7, 6)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+@pytest.mark.parametrize("kind", ["FDK", "matched"])
+def test_expired_wait_leaves_the_volume_unwritten(views, view, accumulate, kind):
+    """Every tile needs the view that does not come, so no voxel may change."""
+    import ctypes as C
+    import torch
+    from tigre_b200 import _native as N, projectors as P
+    geo, ang, _, proj = _case()
+    dproj = torch.from_numpy(proj).cuda()
+    vol = torch.full((64, 64, 64), 7.5, device="cuda")
+    plan = N.Plan(N.checked_geometry(geo, ang), 0)
+
+    def call():
+        N.check(N.lib().tigre_atb_ex(plan.handle, C.c_void_p(dproj.data_ptr()), N.F32, C.c_void_p(vol.data_ptr()), N.F32,
+                                     P.BACKPROJECTORS[kind], 0, views, accumulate, None), "tigre_atb_ex")
+    with N.option(N.OPT_BP_SKIP_COPY, view):
+        call()
+    assert plan.status() & N.STATUS_WAIT_EXPIRED
+    assert bool((vol == 7.5).all())
+    plan = N.Plan(N.checked_geometry(geo, ang), 0)
+    call()                                     # the device is intact
+    assert plan.status() == 0
+    ref = O.atb(proj[:views], geo, ang[:views], kind) + (7.5 if accumulate else 0.0)
+    mx, l2 = G.rel_err(vol.cpu().numpy(), ref)
+    assert mx <= TOL and l2 <= TOL, (mx, l2)
 
 
 def test_expired_wait_fails_the_host_call():
