@@ -211,26 +211,21 @@ int tigre_atb_ex(TigrePlan* plan, const void* d_proj, int pdt, void* d_vol, int 
     const Dims& d = plan->d;
     const int na = a1 - a0;
     int rc = TIGRE_SUCCESS;
-    if (pdt != TIGRE_F32 && (vdt == TIGRE_F32 || vdt == TIGRE_BF16) && bp_tma_supported(plan, TIGRE_F32)) {
-        // 16-bit projections: widened to FP32 (exact) into a pitched copy, then the FP32 patches
+    // the staged kernel reads FP32 patches and writes FP32 or BF16 volumes; FP16 volumes are the general
+    // kernel's, which takes FP16 projections for them
+    const bool staged = bp_tma_supported(plan);
+    if (staged && vdt == TIGRE_F16 && pdt != TIGRE_F16)
+        return fail(TIGRE_ERR_BAD_ASSERT, "unsupported dtype pair for the staged backprojector");
+    if (staged && vdt != TIGRE_F16) {
+        const bool matched = backprojector == TIGRE_BACKPROJ_MATCHED;
+        if (pdt == TIGRE_F32 && d.nU % 4 == 0 && (uintptr_t)d_proj % 16 == 0)
+            return launch_backproject_tma(plan, (const float*)d_proj, d.nU, d_vol, vdt, matched, a0, a1, accumulate, st);
+        // other rows and 16-bit values (widened, exact): a pitched FP32 copy
         const int pitch = (d.nU + 3) / 4 * 4;
         float* s = (float*)plan_scratch(plan, (size_t)na * d.nV * pitch * sizeof(float), st, &rc);
         if (rc) return rc;
         if ((rc = launch_repitch_projections_f32(d_proj, pdt, s, na, d.nV, d.nU, pitch, st))) return rc;
-        return launch_backproject_tma(plan, s, pitch, TIGRE_F32, d_vol, vdt, backprojector == TIGRE_BACKPROJ_MATCHED,
-                                      a0, a1, accumulate, st);
-    }
-    if (bp_tma_supported(plan, pdt)) {
-        const int align = 16 / (int)dtype_size(pdt);
-        if (d.nU % align == 0 && ((uintptr_t)d_proj % 16) == 0)
-            return launch_backproject_tma(plan, d_proj, d.nU, pdt, d_vol, vdt,
-                                          backprojector == TIGRE_BACKPROJ_MATCHED, a0, a1, accumulate, st);
-        const int pitch = (d.nU + align - 1) / align * align;
-        void* s = plan_scratch(plan, (size_t)na * d.nV * pitch * dtype_size(pdt), st, &rc);
-        if (rc) return rc;
-        if ((rc = launch_repitch_projections(d_proj, pdt, s, na, d.nV, d.nU, pitch, st))) return rc;
-        return launch_backproject_tma(plan, s, pitch, pdt, d_vol, vdt, backprojector == TIGRE_BACKPROJ_MATCHED, a0,
-                                      a1, accumulate, st);
+        return launch_backproject_tma(plan, s, pitch, d_vol, vdt, matched, a0, a1, accumulate, st);
     }
     void* s = plan_scratch(plan, (size_t)na * bp_rows(d.nV) * bp_pitch(d.nU) * dtype_size(pdt), st, &rc);
     if (rc) return rc;

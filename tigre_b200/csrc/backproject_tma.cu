@@ -603,16 +603,12 @@ int launch_typed(const CUtensorMap& tm, BPKArgs a, bool matched, bool axial, cud
 
 }  // namespace
 
-bool bp_tma_supported(const TigrePlan* P, int pdt) {
-    if (pdt == TIGRE_F16) return false;
+bool bp_tma_supported(const TigrePlan* P) {
     return P->bp_box_u > 0 && encode_fn() != nullptr;
 }
 
-int launch_backproject_tma(TigrePlan* P, const void* proj, int pitch, int pdt, void* vol, int vdt, int matched,
-                           int a0, int a1, int accumulate, cudaStream_t st) {
-    // FP32 patches only: 16-bit projections are widened first
-    if (pdt != TIGRE_F32 || (vdt != TIGRE_F32 && vdt != TIGRE_BF16))
-        return fail(TIGRE_ERR_BAD_ASSERT, "unsupported dtype pair for the staged backprojector");
+int launch_backproject_tma(TigrePlan* P, const float* proj, int pitch, void* vol, int vdt, int matched, int a0, int a1,
+                           int accumulate, cudaStream_t st) {
     auto enc = encode_fn();
     if (!enc) return fail(TIGRE_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
     const int na = a1 - a0;
@@ -624,7 +620,7 @@ int launch_backproject_tma(TigrePlan* P, const void* proj, int pitch, int pdt, v
     cuuint32_t box[3] = {(cuuint32_t)BU, (cuuint32_t)P->bp_box_v, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
-                     const_cast<void*>(proj), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     const_cast<float*>(proj), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(TIGRE_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     BPKArgs a{};

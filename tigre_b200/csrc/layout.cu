@@ -168,17 +168,7 @@ __global__ void repitch_kernel(const Ts* __restrict__ src, T* __restrict__ dst, 
 
 }  // namespace
 
-int launch_repitch_projections(const void* src, int dtype, void* dst, int nA, int nV, int nU, int pitch,
-                               cudaStream_t st) {
-    const long rows = (long)nA * nV;
-    const long want = (rows * pitch + 255) / 256;
-    const int grid = (int)std::min<long>(want, 148L * 32);
-    TIGRE_DISPATCH_DTYPE(dtype, T, { repitch_kernel<T, T><<<grid, 256, 0, st>>>((const T*)src, (T*)dst, nU, pitch, rows); });
-    TIGRE_LAUNCHED();
-    return TIGRE_SUCCESS;
-}
-
-// 16-bit projections widened to FP32 on the way (exact), same pitching as above
+// FP32 rows of `pitch` elements, zeros behind nU; 16-bit values widen exactly
 int launch_repitch_projections_f32(const void* src, int dtype, float* dst, int nA, int nV, int nU, int pitch,
                                    cudaStream_t st) {
     const long rows = (long)nA * nV;

@@ -191,11 +191,9 @@ int launch_conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw
 int launch_backproject(TigrePlan* p, const void* proj_pad, int pdt, void* vol, int vdt, int matched, int a0, int a1,
                        int accumulate, cudaStream_t st);
 
-bool bp_tma_supported(const TigrePlan* p, int pdt);
-int launch_backproject_tma(TigrePlan* p, const void* proj, int pitch, int pdt, void* vol, int vdt, int matched,
-                           int a0, int a1, int accumulate, cudaStream_t st);
-int launch_repitch_projections(const void* src, int dtype, void* dst, int nA, int nV, int nU, int pitch,
-                               cudaStream_t st);
+bool bp_tma_supported(const TigrePlan* p);
+int launch_backproject_tma(TigrePlan* p, const float* proj, int pitch, void* vol, int vdt, int matched, int a0, int a1,
+                           int accumulate, cudaStream_t st);
 
 // padded projection pitch and row count used by the backprojector
 __host__ __device__ inline long bp_pitch(int nU) { return (long)nU + 3; }
