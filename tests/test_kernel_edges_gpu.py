@@ -515,3 +515,37 @@ def test_convolution_under_saved_tensor_hooks():
     for a, b, bar in zip(got, want, (2.5e-3, 1e-5, 1e-5)):     # bars of test_convolution_and_its_gradients
         assert float((a - b).norm() / b.norm()) < bar
 
+
+@pytest.mark.parametrize("D,H,W", [(4, 16, 8), (6, 18, 10), (9, 7, 23), (8, 4, 4)])
+@pytest.mark.parametrize("ca,cb,cout", [(16, 48, 32), (64, 16, 16), (32, 32, 64)])
+def test_convolution_of_a_pair(D, H, W, ca, cb, cout):
+    """Two inputs where they are: the bits of the convolution of their concatenation."""
+    import torch
+    from tigre_b200 import _native as N
+    g = torch.Generator(device="cuda")
+    g.manual_seed(12)
+    L, p = N.lib(), lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    xa = torch.randn((D, H, W, ca), device="cuda", generator=g).bfloat16()
+    xb = torch.randn((D, H, W, cb), device="cuda", generator=g).bfloat16()
+    w = (0.1 * torch.randn((cout, 27 * (ca + cb)), device="cuda", generator=g)).bfloat16()
+    b = torch.randn(cout, device="cuda", generator=g)
+    x = torch.cat([xa, xb], dim=-1)
+    y, ref = (torch.empty((D, H, W, cout), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    n = 27 * (ca + cb) * cout
+    col = torch.full((n + 64,), 7.0, device="cuda").bfloat16()
+    assert L.tigre_conv3d_fwd_pair_ok(D, H, W, ca, cb, cout) == 1
+    N.check(L.tigre_conv3d_fwd_pair(p(xa), ca, p(xb), cb, p(w), p(b), p(y), D, H, W, cout, 1, p(col), None), "pair")
+    assert bool((col[n:] == 7.0).all())
+    N.check(L.tigre_conv3d_fwd(p(x), p(w), p(b), p(ref), None, D, H, W, ca + cb, cout, 1, p(col), None), "fwd")
+    assert torch.equal(y, ref) and bool(ref.any())
+
+
+@pytest.mark.parametrize("d,h,w,c", [(1, 1, 1, 8), (3, 5, 7, 24), (16, 17, 9, 16)])
+def test_upsampling(d, h, w, c):
+    import torch
+    from tigre_b200 import _native as N
+    x = torch.arange(d * h * w * c, device="cuda").remainder(251).view(d, h, w, c).bfloat16()
+    out = torch.empty((2 * d, 2 * h, 2 * w, c), dtype=torch.bfloat16, device="cuda")
+    N.check(N.lib().tigre_unet_up2(C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr()), 2 * d, 2 * h, 2 * w, c, None), "up2")
+    assert torch.equal(out, x.repeat_interleave(2, 0).repeat_interleave(2, 1).repeat_interleave(2, 2))
+
