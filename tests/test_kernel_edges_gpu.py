@@ -104,6 +104,24 @@ def test_siddon_cell_lists(xy, nv, mode):
     _close(got.cpu().numpy(), O.ax(vol, geo, ang.astype(np.float32), "Siddon"))
 
 
+@pytest.mark.parametrize("nv", [31, 64, 70, 128, 129, 250, 257])
+@pytest.mark.parametrize("mode", ["cone", "parallel"])
+def test_siddon_rows_per_thread(nv, mode):
+    """A thread takes 2, 4 or 8 rows by the scan's size; a ray's arithmetic does not depend on it.  Columns and
+    views that fill the chip against one view at a time (two rows a thread), bit for bit."""
+    import torch
+    from tigre_b200 import projectors as P
+    shape = (24, 17, 19)
+    geo = _geo(shape, (nv, 60), 40.0 / nv, offsets=True, mode=mode)
+    geo.dDetector = np.array((40.0 / nv, 0.6))
+    geo.sDetector = geo.nDetector * geo.dDetector
+    plan = _plan(geo, G.angles(75))
+    vol = torch.from_numpy(np.random.default_rng(nv).random(shape, dtype=np.float32)).cuda()
+    got = P.ax(vol, plan, "Siddon")
+    one = torch.cat([P.ax(vol, plan, "Siddon", angle_range=(i, i + 1)) for i in range(75)])
+    assert torch.equal(got, one) and float(got.max()) > 1.0
+
+
 @pytest.mark.parametrize("nz,vox", [(20, 0.1), (20, 0.3), (24, 1.1)])
 @pytest.mark.parametrize("nv", [5, 65, 257])
 def test_siddon_row_beside_a_slice_plane(nz, vox, nv):

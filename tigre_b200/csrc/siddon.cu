@@ -25,7 +25,8 @@
 
 #include <cstdlib>
 
-#include <utility>
+#include <algorithm>
+#include <tuple>
 
 #include "tigre_internal.h"
 
@@ -772,20 +773,24 @@ int launch_siddon_cells(TigrePlan* P, const float* vol_z, void* proj, int pdt, i
     a.proj = proj;
     a.zpad = P->cells_zpad;
     const int nv = P->d.nV;
-    // Rows per thread: 8, 4 or 2, whichever walks the detector's height at the least cost.  A warp of 4
-    // rows per thread costs 0.56 of one of 8, and one of 2 costs 0.58 of one of 4 (180 views of 256^2:
-    // 986 us with 8 rows, 1112 with 4; 100 of 128^2: 111 with 4, 129 with 2).
-    int R = 8, least = INT32_MAX;
-    for (const auto& [rows, cost] : {std::pair<int, int>{8, 100}, {4, 56}, {2, 33}}) {
-        const int total = (nv + 32 * rows - 1) / (32 * rows) * cost;
-        if (total < least) { least = total; R = rows; }
+    const int na = a1 - a0;
+    // Rows per thread: 8, 4 or 2, whichever takes least.  A warp of them costs an SM 100, 54 or 33 units, in warps
+    // enough to fill it; fewer take their latency, 1700, 1100 or 900.  The measured best or within 3 % of it
+    // over 227 scans of 48^3 to 256^3, 33 to 600 rows and 1 to 180 views (us with 2 | 4 | 8 rows): 100^3, 128 rows,
+    // 3 views 41 | 45 | 61, 163 views 313 | 268 | 471; 256^3, 197 rows, 1 view 148 | 160 | 223, 60 views
+    // 1434 | 1206 | 1159.
+    int R = 8;
+    double least = 1e300;
+    for (const auto& [rows, cost, idle] : {std::tuple<int, double, double>{8, 100, 1700}, {4, 54, 1100}, {2, 33, 900}}) {
+        const double warps = (double)P->d.nU * na * ((nv + 32 * rows - 1) / (32 * rows)) / 148.0;
+        const double t = std::max(idle, cost * warps);
+        if (t < least) { least = t; R = rows; }
     }
     // the copy within one 4 GB-aligned window: its addresses share their high word
     const uintptr_t first = (uintptr_t)vol_z;
     const uintptr_t last = first + (size_t)P->d.nX * P->d.nY * (P->d.nZ + 2 * a.zpad) * sizeof(float) - 1;
     const bool window = first >> 32 == last >> 32;
     const int vtile = 64;   // flat between 32 and 128 views at 512^3 / 1024x768
-    const int na = a1 - a0;
     const int nug = (P->d.nU + kCellWarps - 1) / kCellWarps, nbands = (nv + 32 * R - 1) / (32 * R);
     const long max_views = std::max(1L, (long)INT32_MAX / ((long)nug * nbands));
     for (long c = 0; c < na; c += max_views) {
