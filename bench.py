@@ -521,14 +521,13 @@ def main():
     atb_launch = t_atb / args.steps
     if ax_launch >= atb_launch:
         alg = nseg * 4 + rays * 4           # one voxel gather per Siddon segment + one output write per ray
-        rpt = 8 if NV >= 512 else (4 if NV >= 256 else 2)   # rows per thread, as the launcher picks
-        roof = {"kernel": "siddon_cells_kernel<float,float,%d>" % rpt, "bound": "hbm",
+        roof = {"kernel": "siddon_cells_kernel", "bound": "hbm",
                 "achieved": alg / ax_launch / 1e9, "alg_bytes_per_launch": alg,
                 "traffic": _scaled_traffic("siddon", NA), "traffic_source": TRAFFIC_SOURCE,
                 "binding": _binding("siddon", ax_launch)}
     else:
         alg = upd * 4 * 4 + math.prod(NVOX) * 4   # 4 bilinear taps per update + one volume write
-        roof = {"kernel": "bp_tma_kernel<float,float,true,true>", "bound": "hbm",
+        roof = {"kernel": "bp_tma_kernel", "bound": "hbm",
                 "achieved": alg / atb_launch / 1e9, "alg_bytes_per_launch": alg,
                 "traffic": _scaled_traffic("bp", NA), "traffic_source": TRAFFIC_SOURCE,
                 "binding": _binding("bp", atb_launch)}
@@ -597,7 +596,7 @@ TRAFFIC_SOURCE = ("dram__bytes_read.sum + dram__bytes_write.sum of a single-pass
 # instructions and shared-memory wavefronts per view of the launch.  The Siddon kernel's DRAM
 # traffic is 0.6 % of its algorithmic bytes: it is bound by instruction issue and on-chip load
 # latency; the backprojector reads its taps from shared memory: bound by shared wavefronts and issue.
-PROFILED = {"siddon": {"warp_inst_per_view": 5.401e9 / 36, "source": "profiles/siddon_cells_512cube_36views.txt"},
+PROFILED = {"siddon": {"warp_inst_per_view": 5.596e9 / 36, "source": "profiles/siddon_cells_512cube_36views.txt"},
             "bp": {"warp_inst_per_view": 2.949e9 / 36, "wavefronts_per_view": 7.605e8 / 36,
                    "ideal_wavefronts_per_view": 512 ** 3 * 4 / 32,
                    "source": "profiles/bp_tma_matched_512cube_36views.txt"}}

@@ -24,7 +24,7 @@ def _ref_weights(w, cin, cout):
                                             # tcgen05 path: Cin % 8 == 0 and Cout % 16 == 0, N tiles 16..128
                                             ((8, 6, 10), 16, 16), ((7, 9, 11), 8, 32), ((9, 8, 7), 48, 48),
                                             ((6, 6, 6), 24, 64), ((5, 7, 9), 16, 128), ((3, 4, 5), 64, 192),
-                                            # halo-tile kernel: Cin % 16 == 0, W % 8 == 0, H % 16 == 0
+                                            # halo-tile kernel (Cin and Cout multiples of 16), whole tiles: W % 8 == 0, H % 16 == 0
                                             ((4, 16, 8), 16, 16), ((8, 32, 16), 32, 32), ((6, 16, 24), 48, 16),
                                             ((4, 16, 8), 16, 64), ((2, 16, 8), 64, 128), ((2, 16, 16), 32, 192),
                                             ((5, 16, 8), 96, 32)])

@@ -396,10 +396,12 @@ __global__ void __launch_bounds__(128, 6) siddon_columns_kernel(SiddonArgs p) {
 //  * WINDOW: where the copy lies inside one 4 GB-aligned window (the host looks), an address is
 //    kept per row whose low word alone moves; otherwise it is a 64-bit add per load.
 // Measured (us, projection alone; before: no list, two sets of cell registers, 64-bit addresses):
-// 64^3 100 views of 128^2 147 -> 98, 128^3 180 of 256^2 1370 -> 986, 256^3 90 of 512^2 4439 -> 3667,
-// 512^3 36 of 1024x768 10870 -> 8847.  At 256^3 the multi-cycle packed pipe is 67 % busy, the issue
-// slots 58 %, L1 hits 80 %; a warp waits for loads most.  Not faster: prefetching the columns into L1
-// (3905), 20 resident warps at 96 registers (6371, spills), the adds moved to the integer pipe (3737).
+// 64^3 100 views of 128^2 143 -> 97, 128^3 180 of 256^2 1363 -> 1014, 256^3 90 of 512^2 4399 -> 3721,
+// 512^3 720 of 1024x768 204900 -> 169300 (3 % more without the window).  A warp waits for loads most, then
+// for the packed pipe.  With z measured from the ray's first plane the crossing takes one packed operation
+// less (165600), but a row beside a slice plane then reads the other slice.  Not faster, measured in that form
+// at 256^3 (3667): prefetching the columns into L1 (3905), 20 resident warps at 96 registers (6371,
+// spills), the adds moved to the integer pipe (3737).
 constexpr int kCellWarps = 4;                  // warps (neighbouring detector columns) per block
 constexpr int kListCells = 32;                 // cells per list: one x and one y crossing per lane
 constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23

@@ -211,9 +211,10 @@ def _make_unet_class():
 
         @T.no_grad()
         def infer(self, vol):
-            """The forward pass with this library's fused kernels: first and last convolutions
-            on the CUDA cores (one input / one output channel), the others on the tensor-core
-            convolution, pooling and upsampling+concatenation in one pass each."""
+            """The forward pass with this library's kernels: the first and last convolutions (one
+            input / one output channel) in FP32, the others on the tensor cores, pooling and
+            upsampling in one pass each; the decoder's convolutions read the upsampled level and the
+            skip connection where they are, or a concatenated copy where they cannot."""
             L = N.lib()
             st = _stream(vol)
             vol = vol.float().contiguous()
