@@ -304,7 +304,9 @@ int tigre_tv_denoise_ex(const float* d_src, float* d_dst, long nx, long ny, long
     if (work_floats < tigre_tv_denoise_work_floats(nx, ny, nz))
         return fail(TIGRE_ERR_BAD_ASSERT, "TV denoising: work space too small");
     cudaStream_t st = (cudaStream_t)stream;
-    if (work_floats >= tigre_tv_denoise_fused_floats(nx, ny, nz))
+    // a warp of the one-pass form takes four rows: of a single one three are idle (512 x 1 x 512, 6 iterations 88 us
+    // against 78 in two passes)
+    if (ny > 1 && work_floats >= tigre_tv_denoise_fused_floats(nx, ny, nz))
         return fused_denoise(d_src, d_dst, ProxDims{(int)nx, (int)ny, (int)(nz + 2), 1.f / sx, 1.f / sy, 1.f / sz},
                              lambda, max_iter, d_work, st);
     const long plane = nx * ny, n = plane * (nz + 2);
