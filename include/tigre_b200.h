@@ -310,7 +310,7 @@ long long tigre_conv3d_bwd_weight_work(long D, long H, long W, long Cin, long Co
 /* Forward path of tigre_conv3d_fwd (and of the data gradient): 3 (default) the tcgen05 halo-tile
  * kernel -- one TMA load of a zero-padded input tile per 16 input channels, the 27 taps as
  * shifted shared-memory operand descriptors, TMEM accumulators -- wherever Cin % 16 == 0 and
- * Cout % 16 == 0 (<= 192), else mode 2; when Cin % 8 == 0 and
+ * Cout % 16 == 0 (<= 192), but for volumes so thin or small that another is faster, else mode 2; when Cin % 8 == 0 and
  * Cout % 16 == 0: 0 the warp-level implicit GEMM, 1 the tcgen05 implicit GEMM with per-step
  * gathers, 2 that kernel for narrow layers (Cin <= 16 or Cout == 16) and the warp-level one
  * otherwise.  Returns the old mode. */

@@ -567,3 +567,29 @@ def test_upsampling(d, h, w, c):
     N.check(N.lib().tigre_unet_up2(C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr()), 2 * d, 2 * h, 2 * w, c, None), "up2")
     assert torch.equal(out, x.repeat_interleave(2, 0).repeat_interleave(2, 1).repeat_interleave(2, 2))
 
+
+@pytest.mark.parametrize("D,H,W,halo", [(200, 1, 200, 0), (200, 2, 200, 0), (40, 3, 300, 0), (200, 5, 200, 1), (50, 50, 50, 1),
+                                        (96, 1, 1, 1), (5, 16, 8, 1), (200, 200, 1, 0)])
+def test_convolution_of_thin_volumes(D, H, W, halo):
+    """Volumes much thinner than a tile keep the kernels that gather voxels; both give the FP64 convolution.
+    Bars of test_convolution_and_its_gradients."""
+    import torch
+    from tigre_b200 import _native as N
+    g = torch.Generator(device="cuda")
+    g.manual_seed(13)
+    L, p = N.lib(), lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    cin, cout = 32, 48
+    assert L.tigre_conv3d_fwd_pair_ok(D, H, W, 16, 16, cout) == halo
+    x = torch.randn((D, H, W, cin), device="cuda", generator=g).bfloat16()
+    w = (0.1 * torch.randn((cout, 27 * cin), device="cuda", generator=g)).bfloat16()
+    dy = torch.randn((D, H, W, cout), device="cuda", generator=g).bfloat16()
+    y, dx = torch.empty_like(dy), torch.empty((D, H, W, cin), device="cuda")
+    col = torch.empty(2 * 27 * D * H * W * cin, dtype=torch.bfloat16, device="cuda")
+    N.check(L.tigre_conv3d_fwd(p(x), p(w), None, p(y), None, D, H, W, cin, cout, 0, p(col), None), "fwd")
+    N.check(L.tigre_conv3d_bwd_data(p(dy), p(w), p(dx), D, H, W, cin, cout, p(col), None), "bwd_data")
+    ref = _conv64(x, w, cout)[0].permute(1, 2, 3, 0)
+    assert float((y.double() - ref).norm() / ref.norm()) < 2.5e-3
+    wt = w.view(cout, 27, cin).flip(1).permute(2, 1, 0).reshape(cin, 27 * cout)
+    ref = _conv64(dy, wt, cin)[0].permute(1, 2, 3, 0)
+    assert float((dx.double() - ref).norm() / ref.norm()) < 1e-5
+

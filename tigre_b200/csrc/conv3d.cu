@@ -509,7 +509,7 @@ int grid_for_conv(long n) { return (int)std::min<long>((n + 255) / 256, 148L * 3
 using namespace tigre;
 
 // Forward path selection: 3 (default) = the tcgen05 halo-tile kernel (conv3d_tc.cu) wherever its
-// shape rules hold (Cin % 16 == 0, Cout % 16 == 0), else mode 2;
+// shape rules hold (Cin % 16 == 0, Cout % 16 == 0) and it is the faster one (halo_fwd), else mode 2;
 // 0 = warp-level implicit GEMM, 1 = tcgen05 implicit GEMM with per-step gathers, 2 = that
 // tcgen05 kernel for narrow layers (Cin <= 16 or Cout == 16) and the warp-level one for wider ones.
 static std::atomic<int> g_conv_tcgen05{3};
@@ -566,6 +566,28 @@ long long tigre_conv3d_bwd_weight_work(long D, long H, long W, long Cin, long Co
     return std::max(8L, 2 * conv_wgrad_work(D, H, W, Cin, Cout));
 }
 
+// Where the halo-tile kernel is the faster one.  It computes whole tiles of 8 x 16 (x, y), so thin volumes pay for
+// `waste` times their voxels; sizes in whole tiles always take it.  Measured (us, halo | the kernels below it):
+// forward, 32 -> 32 channels: 100 x 4 x 100 (waste 4.2) 31 | 34, 200 x 1 x 200 (16) 81 | 31, but 96 x 1 x 1 (128, one round of
+// blocks) 15 | 17; 16 -> 16 channels, whose gathering kernel arranges no weights: 12^3 14.8 | 13.2, 25^3 14.9 | 13.9,
+// 33 x 7 x 126 15.5 | 20.4.  Data gradient into FP32 against the GEMM: 16 x 17 x 9, 64 -> 64 33 | 30, 25^3 35 | 149,
+// 96 x 1 x 1, 32 -> 32 15 | 10.
+static double halo_waste(long H, long W) {
+    return (double)((H + 15) / 16 * 16) * (double)((W + 7) / 8 * 8) / ((double)H * (double)W);
+}
+static bool halo_fwd(long D, long H, long W, long Cin, long Cout) {
+    if (!conv_tc_halo_supported(D, H, W, Cin, Cout)) return false;
+    if (H % 16 == 0 && W % 8 == 0) return true;
+    if (Cin == 16 && D * H * W < 20000) return false;
+    const long tiles = (H + 15) / 16 * ((W + 7) / 8) * ((D + 3) / 4);
+    return halo_waste(H, W) <= 4.5 || tiles <= 148;
+}
+static bool halo_bwd_data(long D, long H, long W, long Cin, long Cout) {
+    if (!conv_tc_halo_supported(D, H, W, Cout, Cin)) return false;
+    if (H % 16 == 0 && W % 8 == 0) return true;
+    return halo_waste(H, W) <= 8.0 && (Cout <= 32 || 54.0 * Cin * Cout * (double)(D * H * W) >= 6e8);
+}
+
 int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void* d_y_bf16, float* d_y_f32, long D,
                      long H, long W, long Cin, long Cout, int relu, void* d_col, void* stream) {
     TIGRE_NVTX("tigre_conv3d_fwd");
@@ -578,7 +600,7 @@ int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void
     // the tcgen05 kernels store 16 bytes at a time; the others take any output address
     const bool y_aligned = (((uintptr_t)d_y_bf16 | (uintptr_t)d_y_f32) & 15) == 0;
     if (tc_mode == 3 && ((uintptr_t)d_x & 15) == 0 && ((uintptr_t)d_col & 15) == 0 && y_aligned &&
-        27L * Cin * Cout <= tigre_conv3d_col_elems(D, H, W, Cin) && conv_tc_halo_supported(D, H, W, Cin, Cout))
+        27L * Cin * Cout <= tigre_conv3d_col_elems(D, H, W, Cin) && halo_fwd(D, H, W, Cin, Cout))
         return launch_conv_tc_halo((const __nv_bfloat16*)d_x, nullptr, 0, (const __nv_bfloat16*)d_w, d_bias,
                                    (__nv_bfloat16*)d_y_bf16, d_y_f32, D, H, W, Cin, Cout, relu, 0,
                                    (__nv_bfloat16*)d_col, status, st);
@@ -632,7 +654,7 @@ int tigre_conv3d_fwd(const void* d_x, const void* d_w, const float* d_bias, void
 // is; 0 where it cannot (the caller then concatenates).
 int tigre_conv3d_fwd_pair_ok(long D, long H, long W, long Ca, long Cb, long Cout) {
     return D > 0 && H > 0 && W > 0 && Ca > 0 && Cb > 0 && Ca % 16 == 0 && Cb % 16 == 0 && g_conv_tcgen05.load() == 3 &&
-           Cout <= D * H * W && conv_tc_halo_supported(D, H, W, Ca + Cb, Cout);
+           Cout <= D * H * W && halo_fwd(D, H, W, Ca + Cb, Cout);
 }
 
 int tigre_conv3d_fwd_pair(const void* d_xa, long Ca, const void* d_xb, long Cb, const void* d_w, const float* d_bias,
@@ -655,7 +677,7 @@ int tigre_conv3d_bwd_data(const void* d_dy, const void* d_w, float* d_dx, long D
     const long M = D * H * W, K = 27 * Cin;
     cudaStream_t st = (cudaStream_t)stream;
     if (g_conv_tcgen05.load() == 3 && (((uintptr_t)d_dy | (uintptr_t)d_dx | (uintptr_t)d_dcol) & 15) == 0 &&
-        Cout <= 2 * M && conv_tc_halo_supported(D, H, W, Cout, Cin)) {   // d_dcol holds the arranged weights
+        Cout <= 2 * M && halo_bwd_data(D, H, W, Cin, Cout)) {   // d_dcol holds the arranged weights
         // the data gradient is the convolution of dy with the tap-flipped, channel-transposed
         // weights: the halo kernel, FP32 output, no im2col (d_dcol holds the arranged weights)
         return launch_conv_tc_halo((const __nv_bfloat16*)d_dy, nullptr, 0, (const __nv_bfloat16*)d_w, nullptr, nullptr, d_dx, D,
